@@ -17,6 +17,7 @@ HOST (host copy newer), DEVICE (device copy newer), BOTH.
   pyop2/device.py:257-303) and launches colour by colour.
 """
 
+import copy
 import ctypes as C
 import hashlib
 import os
@@ -633,9 +634,11 @@ class Mat(DeviceDataMixin, base.Mat):
         base.Mat.__init__(self, sparsity, dtype, name)
         self._state = DEVICE_UNALLOCATED
         self._vals = None
-        # True while every value is known to be zero (fresh or zero()ed): the
-        # two-phase reduction then need not read the values
-        self._is_zero = True
+        # every value is known to be zero (fresh or zero()ed): an assembly
+        # that owns the values then need not read them.  True; or the graph
+        # being recorded, when the zeroing is recorded in it and so holds for
+        # what the same graph does next, not for anything run now
+        self._zeroed = True
 
     def _device_values(self):
         if self._vals is None:
@@ -667,7 +670,21 @@ class Mat(DeviceDataMixin, base.Mat):
 
     def zero(self):
         self._device_values().memset(0)
-        self._is_zero = True
+        graph = _state.get('capturing')
+        self._zeroed = graph if graph else True
+        if graph:
+            graph.note_mat(self)
+
+    def _known_zero(self):
+        return self._zeroed is (_state.get('capturing') or True)
+
+    def _written(self):
+        """The values may be anything from here on; a graph that records the
+        write may repeat it whenever it is launched."""
+        self._zeroed = False
+        graph = _state.get('capturing')
+        if graph:
+            graph.note_mat(self)
 
     def zero_rows(self, rows, diag_val):
         """Zero the given rows except the diagonal, set to diag_val.
@@ -684,7 +701,7 @@ class Mat(DeviceDataMixin, base.Mat):
             raise IndexError("zero_rows: row %d outside [0, %d)" % (bad, nrows))
         rows = rows.astype(np.int32)
         vals = self._device_values()
-        self._is_zero = False
+        self._written()
         call("op2b_mat_zero_rows", vals.ptr, self._sparsity._d_rowptr, self._sparsity._d_colidx,
              nrows, rows.ctypes.data_as(C.POINTER(C.c_int32)), rows.size, float(diag_val),
              self.dtype.itemsize, 0)
@@ -1116,6 +1133,114 @@ def _incidence(m):
     return inc
 
 
+class RowBlocks(object):
+    """Row blocks of a loop that increments through one Map
+    (op2b_row_blocks_build)."""
+
+    @classmethod
+    def of(cls, rmap, region, stage_maps, ids, sparsity=None, cmap=None):
+        """The row blocks of increments through ``rmap`` (into ``sparsity``'s
+        entries with columns ``cmap``), with the elements' ``ids`` for loops
+        that need them, built at first use and kept with the Map; None where
+        the form does not apply."""
+        tables = rmap.__dict__.setdefault("_row_block_tables", {})
+        key = (region, tuple(id(m) for m in stage_maps), ids, id(sparsity), id(cmap))
+        hit = tables.get(key)
+        if hit is None:
+            ns = len(stage_maps)
+            smap = (C.c_uint64 * max(ns, 1))(*[m._to_device().ptr for m in stage_maps])
+            sar = (C.c_int32 * max(ns, 1))(*[m.dim for m in stage_maps])
+            h = C.c_uint64()
+            call("op2b_row_blocks_build", rmap._to_device().ptr, rmap.dim, rmap.iterset.size,
+                 rmap.dataset.size, region, cmap._to_device().ptr if cmap is not None else 0,
+                 cmap.dim if cmap is not None else 1, sparsity._d_rowptr if sparsity else 0,
+                 sparsity._d_colidx if sparsity else 0, ns, smap, sar, int(ids), 0, C.byref(h))
+            # the Maps and the Sparsity stay alive as long as their ids are keys
+            hit = tables[key] = (cls(h.value) if h.value else None, list(stage_maps), cmap, sparsity)
+        return hit[0]
+
+    def __init__(self, handle):
+        self._handle = handle
+        nb, mi, mp = C.c_int32(), C.c_int32(), C.c_int32()
+        mt = (C.c_int32 * 4)()
+        d, pkt = C.c_uint64(), C.c_uint64()
+        call("op2b_row_blocks_info", handle, C.byref(nb), C.byref(mi), C.byref(mp), mt, C.byref(d),
+             C.byref(pkt))
+        self.nblocks, self.max_items, self.max_packet = nb.value, mi.value, mp.value
+        self.max_targets = list(mt)
+        # parameter values of a row block stub
+        self.vals = {"rb_dir": d.value, "rb_pkt": pkt.value, "rb_blocks": self.nblocks}
+
+    def __del__(self):
+        try:
+            if self._handle and _state['init']:
+                _lib._lib.op2b_row_blocks_free(self._handle)
+        except Exception:
+            pass
+
+
+# threads per CTA of the row block stubs, and bytes of contributions a block
+# aims at per incremented object (its region's elements times the bytes of one
+# element)
+_ROWBLK_THREADS = 128
+_ROWBLK_BYTES = 15360
+
+
+# contributions a launch adds, below which the row blocks' phases cost as much
+# as the reductions they save (P1 256 x 256, 1.2 million: 13.0 to 15.9 us by the
+# partition, 14.3 with reductions; P2 181 x 181, 2.4 million: 28.7 against 36.1)
+_ROWBLK_MIN = 3 << 19
+
+# runs of a bound loop before its row blocks are built: the build takes what 30
+# (P2) to 80 (P1) runs then save, and the element form needs only the slot table,
+# so a loop that runs a few times keeps that one
+_ROWBLK_RUNS = 32
+# what ran within so many loops before a graph capture is taken to be what it
+# will record, and gets its row blocks before it
+_ROWBLK_RECENT = 256
+_runs = [0]
+
+
+def row_block_spec(spec, specs, maps, mats, kahan=False):
+    """(the loop's spec in the row block form, its RowBlocks), or None where
+    that form does not run the loop."""
+    kind = codegen.rowblk_capable(spec) if spec.mode in ("atomic", "lma", "staged") else None
+    if kind is None or (kind == "mat" and any(m.sparsity is not mats[0].sparsity for m in mats)):
+        return None
+    w = next(s for s in specs if s.access == "INC" and s.kind != "gbl")
+    reads = _region_layout([s for s in specs if s.access == "READ"], maps)
+    if len(reads["stage_arity"]) > 4:
+        return None
+    new = copy.copy(spec)
+    new.mode, new.block_size = "rowblk", _ROWBLK_THREADS
+    incs = [] if kind == "mat" else sorted({(s.slot, s.mslot, s.ctype, s.cdim) for s in specs
+                                            if s.access == "INC" and s.kind != "gbl"})
+    new.rowblk = {"kind": kind, "ra": w.arity, "ca": w.carity if kind == "mat" else 1,
+                  "kahan": bool(kahan), "map_stage": reads["map_stage"],
+                  "stage_arity": reads["stage_arity"], "read_pairs": reads["read_pairs"],
+                  "incs": incs}
+    new.mat_slots, new.mat_alias, new.mat_slots_rel, new.itspace_split = False, (), False, None
+    new.mat_per_entry, new.region, new.gathered = False, None, ()
+    rmap = maps[w.mslot]
+    stage_maps = [maps[k] for k in reads["stage_maps"]]
+    ids = any(s.kind == "direct" for s in specs)
+    # bytes one element adds to the largest contribution array
+    one = max(w.arity * new.rowblk["ca"] * c * codegen._CSIZE[t]
+              for t, c, _, _ in codegen._rowblk_targets(new))
+    region = max(16, min(512, _ROWBLK_BYTES // one))
+    if kind == "mat":
+        sp = mats[0].sparsity
+        if sp._dims != (1, 1):
+            return None
+        rb = RowBlocks.of(rmap, region, stage_maps, ids, sp, maps[w.cmslot])
+    else:
+        rb = RowBlocks.of(rmap, region, stage_maps, ids)
+    if rb is None or codegen.rowblk_smem(new, rb.max_items, rb.max_packet, rb.max_targets) > \
+            _state['smem_optin']:
+        return None
+    return new, rb
+
+
 # --------------------------------------------------------------- JIT cache
 _MODULES = {}
 
@@ -1544,6 +1669,13 @@ def _sync_consts(mod, consts):
     mod.const_stamp = stamp
 
 
+def _default_mat_form():
+    """The Mat options leave the form of an assembly to the backend (a
+    caller who sets one of them asks for the element form it tunes)."""
+    return (cfg.cfg['mat_slots'] and cfg.cfg['mat_per_entry'] and not cfg.cfg['mat_slots_rel']
+            and cfg.cfg['itspace_split'] == 'auto')
+
+
 class _StagedTooLarge(Exception):
     """The staged form of a loop needs more shared memory per CTA than the
     device has: the loop is bound in the atomic form instead."""
@@ -1553,9 +1685,10 @@ class _BoundLoop(object):
     """Everything about a par_loop that does not change between calls with
     the same objects: generated stub, plan, parameter block."""
 
-    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None):
+    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None, rows=False):
         # nelem: bind to the set's first nelem elements only (the core of a
-        # partitioned set, run in the staged form)
+        # partitioned set, run in the staged form); rows: in the row block form
+        # if it runs the loop
         info = loop_spec(loop, inc_mode=inc_mode, owner_mode=owner_mode, size=nelem)
         spec = info['spec']
         specs = info['specs']
@@ -1563,6 +1696,29 @@ class _BoundLoop(object):
         stages, races, indirect = info['stages'], info['races'], info['indirect']
         iterset = info['iterset']
         args = loop.args
+        self.row_blocks = None
+        self._runs, self._last_run = 0, -_ROWBLK_RECENT
+        # Mat assembly by the owners of the rows (see codegen._rowblk_body): at
+        # once in place of the two-phase form, whose own tables cost as much to
+        # build; else when the loop has run often enough (see run)
+        w = next((s for s in specs if s.kind == "mat"), None)
+        self._rows_later = bool(
+            w is not None and nelem is None and inc_mode is None and not _partitioned(iterset)
+            and (spec.mode == "lma" or (spec.mode == "atomic" and _default_mat_form()))
+            and iterset.size * w.arity * w.carity >= _ROWBLK_MIN and codegen.rowblk_capable(spec))
+        if self._rows_later and (rows or spec.mode == "lma"):
+            self._rows_later = False
+            try:
+                form = row_block_spec(spec, specs, maps, mats,
+                                      kahan=spec.mode == "lma" and cfg.cfg['kahan'])
+            except DeviceError as e:          # no memory for the tables
+                debug("row blocks of %s: %s" % (loop.kernel.name, e))
+                form = None
+            if form is not None:
+                spec, self.row_blocks = form
+                info['block_size'] = spec.block_size
+        # what promotion needs beside the arguments of the call
+        self._again = (loop.kernel, loop.it_space) if self._rows_later else None
         self.spec = spec
         self.nelem = iterset.size if nelem is None else int(nelem)
         self.core_loop = None
@@ -1679,6 +1835,13 @@ class _BoundLoop(object):
             self.module.ensure_smem(self.launch_smem)
             self.grid = rp.nblocks
             self.max_grid = max(1, rp.nblocks)
+        elif spec.mode == "rowblk":
+            rb = self.row_blocks
+            vals.update(rb.vals)
+            self.launch_smem = codegen.rowblk_smem(spec, rb.max_items, rb.max_packet, rb.max_targets)
+            self.module.ensure_smem(self.launch_smem)
+            occ = max(1, self.module.occupancy(self.module.fn, bs, self.launch_smem))
+            self.grid = self.max_grid = min(rb.nblocks, occ * _state['sm_count'])
         elif spec.mode == "lma":
             # two-phase INC: contribution arrays (phase 1, the stub) and the
             # incidences their reduction walks (phase 2, op2b_lma_reduce)
@@ -1795,11 +1958,16 @@ class _BoundLoop(object):
             else:
                 self._ginit.append(None)
         self._gflag = [0] * len(self._gbl)
+        self._mzero = [0] * len(self.mats)
         self._written = [d for d in self.dats if any(m != "READ" for m in self.dat_access[id(d)])]
         self._reducing = [k for k, (_, _, red) in enumerate(self._gbl) if red]
         n = self.nelem
         self._buf = C.create_string_buffer(self.layout.pack(n, 0, self.range_end, vals),
                                            self.layout.nbytes)
+        if self.row_blocks is not None:
+            # the header's second colour field: room of a packet
+            struct.pack_into("<i", self._buf, codegen.ParamLayout.COL_OFFSET + 4,
+                             self.row_blocks.max_packet)
 
     def run(self, loop, rng=None):
         """Run the loop over its whole set, or over elements [start, end)
@@ -1818,7 +1986,21 @@ class _BoundLoop(object):
         n = self.nelem if rng is None else rng[1] - rng[0]
         trace.append((pre, _capture_tail(), self.accesses + gbl, n))
 
+    def _to_rows(self, args):
+        """Bind again in the row block form (the element form where that
+        does not run the loop)."""
+        kernel, it_space = self._again
+        trace_runs = self._runs
+        _BoundLoop.__init__(self, _Loop(kernel, it_space, args), rows=True)
+        self._buf, self._runs = None, trace_runs
+
     def _run(self, loop, rng=None):
+        _runs[0] += 1
+        if self._rows_later:
+            self._runs += 1
+            self._last_run, self._args = _runs[0], loop.args
+            if self._runs > _ROWBLK_RUNS and not _state.get('capturing'):
+                self._to_rows(self._args)
         if getattr(self, "_buf", None) is None:
             self._prepare(loop)
         for d in self.dats:
@@ -1857,6 +2039,12 @@ class _BoundLoop(object):
         mod = self.module
         if self.consts:
             _sync_consts(mod, self.consts)
+        if self.row_blocks is not None:
+            for j, m in enumerate(self.mats):
+                z = 1 if m._known_zero() else 0
+                if z != self._mzero[j]:
+                    struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), z)
+                    self._mzero[j] = z
         n = self.nelem
         if rng is not None:
             if self.spec.mode not in ("direct", "atomic") or rng[0] < 0 or rng[1] > \
@@ -1890,8 +2078,8 @@ class _BoundLoop(object):
                     # Mat incidences hold contribution indices (OP2B_LMA_MAT_INDEX);
                     # a Mat known to be zero needs no read of its values
                     # (OP2B_LMA_FROM_ZERO)
-                    flags = kahan | 4 | (2 if target._is_zero else 0)
-                    target._is_zero = False
+                    flags = kahan | 4 | (2 if target._known_zero() else 0)
+                    target._written()
                 else:
                     out, flags = target._device.ptr, kahan
                 call("op2b_lma_reduce", out, cdim, inc.ptr, inc.list, ntargets, buf.ptr, n,
@@ -1904,7 +2092,7 @@ class _BoundLoop(object):
             args[self._gbl[k][1]].data._state = DEVICE
         for m in self.mats:
             m._state = DEVICE
-            m._is_zero = False
+            m._written()
 
 
 _ENV = {"gen": None, "key": None}
@@ -1967,6 +2155,13 @@ def _key_kind(t):
     k = "g" if issubclass(t, base.Global) else "m" if issubclass(t, base.Mat) else "d"
     _KEY_KIND[t] = k
     return k
+
+
+class _Loop(object):
+    """Kernel, iteration space and arguments of a loop to bind again."""
+
+    def __init__(self, kernel, it_space, args):
+        self.kernel, self.it_space, self.args = kernel, it_space, args
 
 
 class _Args(object):
@@ -2324,9 +2519,18 @@ class Graph(object):
     def __init__(self):
         self.handle = 0
         self.segments = None
+        self._mats = {}
+
+    def note_mat(self, m):
+        """The graph writes Mat ``m``."""
+        self._mats[id(m)] = weakref.ref(m)
 
     def launch(self):
         call("op2b_graph_launch", self.handle, 0)
+        for ref in self._mats.values():
+            m = ref()
+            if m is not None:
+                m._written()
 
     def close(self):
         """Destroy the executable graph now rather than at collection."""
@@ -2392,6 +2596,15 @@ def _relaxed_exec(graph, trace, small_only=False):
     return h.value, [(acc is not None, d) for (_, _, acc), d in zip(segs, deps)]
 
 
+def _rows_before_capture():
+    """Build the row blocks of the assembly loops that ran just before: a
+    graph is recorded to be replayed, and cannot change its loops' form."""
+    since = _runs[0] - _ROWBLK_RECENT
+    for bl in list(ParLoop._bound_cache.values()):
+        if bl._rows_later and bl._last_run > since:
+            bl._to_rows(bl._args)
+
+
 class capture(object):
     """Record the par_loops issued inside the block into a CUDA graph instead
     of running them::
@@ -2419,9 +2632,10 @@ class capture(object):
         self.small_only = mode == "small"
 
     def __enter__(self):
+        _rows_before_capture()
         self.graph = Graph()
         call("op2b_graph_begin", 0)
-        _state['capturing'] = True
+        _state['capturing'] = self.graph
         _state['trace'] = [] if self.overlap else None
         return self.graph
 

@@ -223,7 +223,7 @@ class LoopInstance(object):
                 hit += 1
         if hit == 0:
             raise ValueError("none of the objects to patch is an argument of the loop")
-        return PatchedInstance(self, bytes(buf))
+        return PatchedInstance(self, bytes(buf), [m for m in self.mats if id(m) not in by_id])
 
     def sync(self):
         """Upload Dats and Globals whose host copy is newer."""
@@ -243,7 +243,7 @@ class LoopInstance(object):
             g._state = b200.DEVICE
         for m in self.mats:
             m._state = b200.DEVICE
-            m._is_zero = False
+            m._written()
 
 
 class PatchedInstance(object):
@@ -251,13 +251,14 @@ class PatchedInstance(object):
     signature with its own parameter block.  Its data lives in raw device
     memory owned by the caller, so there is no host copy to synchronise."""
 
-    __slots__ = ("spec", "key", "size", "params")
+    __slots__ = ("spec", "key", "size", "params", "mats")
     form = "atomic"     # patched instances run the atomic batched form
     plan = None
 
-    def __init__(self, template, params):
+    def __init__(self, template, params, mats):
         self.spec, self.key, self.size = template.spec, template.key, template.size
         self.params = params
+        self.mats = mats          # the template's own Mats the loop still writes
 
     def sync(self):
         pass
@@ -282,6 +283,7 @@ class BatchLoop(object):
         for n, inst in enumerate(self.instances):
             if inst.key != key:
                 raise ValueError("instance %d of the batch has a different loop signature" % n)
+        self._mats = list({id(m): m for i in self.instances for m in i.mats}.values())
         spec = copy.copy(self.instances[0].spec)
         spec.block_size = int(block_size or cfg.cfg['block_size'])
         spec.batch = int(elems_per_thread)
@@ -425,6 +427,8 @@ class BatchLoop(object):
                  self._params, self.layout.nbytes)
         if self.has_fin and self.nsegs:
             call("op2b_launch", self.fin, self.fin_grid, 256, 0, 0, self._params, self.layout.nbytes)
+        for m in self._mats:
+            m._written()
         if sync_host:
             for inst in self.instances:
                 inst.mark()

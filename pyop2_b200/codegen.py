@@ -25,6 +25,7 @@ synchronise per colour).  Per element the stub:
   the device (op2b_device.cuh: op2b_reduce).
 """
 
+import copy
 import os
 import re
 import struct
@@ -75,6 +76,8 @@ class LoopSpec(object):
         # one grid-stride launch, INC args added with atomics
         self.mode = mode or ("plan" if indirect else "direct")
         self.owner = None   # owner-computes description (mode 'owner')
+        # row block form (mode 'rowblk'): see _rowblk_body
+        self.rowblk = None
         # elements per thread of a batched launch (0: not batched); see _batch_body
         self.batch = 0
         # scalar Mats found through scatter-slot tables (op2b_mat_slots_build)
@@ -127,7 +130,7 @@ class LoopSpec(object):
                 tuple(sorted(self.owner.items())) if self.owner else None, self.batch,
                 self.mat_slots, _freeze(self.region), tuple(self.mat_alias),
                 self.mat_per_entry, self.itspace_split, self.direct_unroll,
-                self.mat_slots_rel, tuple(self.gathered))
+                self.mat_slots_rel, tuple(self.gathered), _freeze(self.rowblk))
 
     @property
     def needs_coloring(self):
@@ -162,6 +165,9 @@ class ParamLayout(object):
         if spec.mode == "staged":
             f += ["rg_order", "rg_boff", "rg_tlist", "rg_toff", "rg_tcnt", "rg_loc", "rg_thrcol",
                   "rg_nthrcol"]
+        if spec.mode == "rowblk":
+            f += ["rb_dir", "rb_pkt", "rb_blocks"]
+            f += ["mz%d" % j for j in range(len(spec.mats))]
         for j in range(len(spec.dats)):
             f.append("d%d" % j)
             if spec.dats[j][1]:
@@ -207,7 +213,8 @@ def _struct_decl(spec, layout):
              "inc_order": "const int *",
              "rg_order": "const int *", "rg_boff": "const int *", "rg_tlist": "const int *",
              "rg_toff": "const int *", "rg_tcnt": "const int *", "rg_loc": "const short *",
-             "rg_thrcol": "const int *", "rg_nthrcol": "const int *"}
+             "rg_thrcol": "const int *", "rg_nthrcol": "const int *",
+             "rb_dir": "const int2 *", "rb_pkt": "const uint4 *", "rb_blocks": "op2b_i64 "}
     for n in layout.fields:
         if n in types:
             t = types[n]
@@ -215,6 +222,8 @@ def _struct_decl(spec, layout):
             t = "op2b_i64 "
         elif n.startswith("d"):
             t = "%s *" % spec.dats[int(n[1:])][0]
+        elif n.startswith("mz"):
+            t = "op2b_i64 "
         elif n.startswith("mv"):
             t = "%s *" % spec.mats[int(n[2:])]
         elif n.startswith("lm"):
@@ -286,7 +295,7 @@ def generate(spec):
         return "\n".join(out), layout, batch_stub_names(spec)[0]
     body = {"plan": _indirect_body, "atomic": _atomic_body, "lma": _atomic_body,
             "direct": _direct_body, "owner": _owner_body, "staged": _staged_body,
-            "gather": _gather_body}[spec.mode](spec)
+            "gather": _gather_body, "rowblk": _rowblk_body}[spec.mode](spec)
     w(_enter(body))
     return "\n".join(out), layout, stub_name(spec)
 
@@ -862,13 +871,15 @@ def _staged_element_parts(spec, R, ind, evar):
     decl, pre, post, exprs, adds = [], [], [], [], []
     for n, a in enumerate(spec.args):
         t, c = a.ctype, a.cdim
+        if a.kind == "mat":       # row blocks: the caller's own locals
+            continue
         if a.kind == "gbl":
             exprs.append("g%d_l" % n if a.access == "READ" else "r%d" % n)
             continue
         if a.kind == "direct":
             exprs.append(_direct_row(a, n, evar, pre, post, ind + "  "))
             continue
-        st = R["map_stage"][a.mslot]
+        st = R["map_stage"].get(a.mslot)
         cnt = a.arity if a.kind == "vec" else a.ext
 
         def row_ptr(rowexpr):
@@ -1201,6 +1212,331 @@ def _atomic_element(spec, ind, ranges=None):
     L += _itspace_close(spec, ind)
     L += post
     L += apply
+    return L
+
+
+def rowblk_capable(spec):
+    """Loops the row block form can run: every write is an INC, all of them
+    through one Map -- scalar Mats over their full local tensor (rows on i0,
+    columns on i1, one (row, column) Map pair) or Dats at every index of the
+    Map, each (Dat, index) once -- every other argument is READ, and at most
+    four Maps are read through.  Returns 'mat', 'dat' or None."""
+    mats = [a for a in spec.args if a.kind == "mat"]
+    incs = [a for a in spec.args if a.kind != "mat" and a.access != "READ"]
+    if any(a.access != "INC" or a.kind not in ("ind", "vec", "its") for a in incs):
+        return None
+    if any(a.ctype not in _CSIZE for a in mats + incs):
+        return None
+    if mats:
+        ok = (not incs and len(spec.extents) == 2 and len({a.slot for a in mats}) == len(mats)
+              and all(a.access == "INC" and a.rm * a.cm == 1 and (a.idx, a.cidx) == (0, 1)
+                      and (a.mslot, a.cmslot) == (mats[0].mslot, mats[0].cmslot)
+                      and tuple(spec.extents) == (a.arity, a.carity) for a in mats))
+        return "mat" if ok else None
+    if not incs or len({a.mslot for a in incs}) != 1:
+        return None
+    seen = {}
+    for a in incs:
+        if a.kind == "its" and (len(spec.extents) != 1 or a.idx != 0 or a.ext != a.arity):
+            return None
+        at = [a.idx] if a.kind == "ind" else list(range(a.arity))
+        got = seen.setdefault(a.slot, [])
+        if set(got) & set(at):
+            return None
+        got += at
+    if any(sorted(got) != list(range(incs[0].arity)) for got in seen.values()):
+        return None
+    # an INC Dat read in the same loop would see other blocks' sums
+    if any(a.access == "READ" and a.kind != "gbl" and a.slot in seen for a in spec.args):
+        return None
+    return "dat"
+
+
+def _rowblk_targets(spec):
+    """(ctype, cdim, name of the device array, index of the zero flag or None)
+    per incremented Mat or Dat slot."""
+    if spec.rowblk["kind"] == "mat":
+        return [(spec.mats[j], 1, "p.mv%d" % j, j) for j in range(len(spec.mats))]
+    out = {}
+    for a in spec.args:
+        if a.access == "INC":
+            out[a.slot] = (a.ctype, a.cdim, "p.d%d" % a.slot, None)
+    return [out[j] for j in sorted(out)]
+
+
+def _rowblk_slots(spec):
+    """Mat or Dat slot -> its place in _rowblk_targets."""
+    if spec.rowblk["kind"] == "mat":
+        return {j: j for j in range(len(spec.mats))}
+    return {j: q for q, j in enumerate(sorted({a.slot for a in spec.args if a.access == "INC"}))}
+
+
+def rowblk_smem(spec, max_items, max_packet, max_targets):
+    """Dynamic shared memory of a row block launch: a packet, the staged READ
+    rows, and per incremented object the contributions of a block, [ca][odd
+    number of items], and one place of zeros."""
+    R = spec.rowblk
+    nb = 16 * max_packet + rowblk_rows(spec, max_targets)
+    for ctype, cdim, _, _ in _rowblk_targets(spec):
+        nb += ((((max_items + 1) | 1) * R["ca"] + 1) * cdim * _CSIZE[ctype] + 15) // 16 * 16
+    return nb
+
+
+def rowblk_rows(spec, max_targets):
+    """Bytes of the staged READ rows of a block."""
+    return sum((max_targets[st] * cdim * _CSIZE[ctype] + 15) // 16 * 16
+               for slot, st, ctype, cdim in spec.rowblk["read_pairs"])
+
+
+def _rowblk_parse(spec, ind):
+    """Lines naming the parts of the packet at pk and the staged rows."""
+    R = spec.rowblk
+    L = ["%sconst int NE = (int)pk->x, nshort = (int)pk->y, nlong = (int)pk->z, NI = (int)pk->w;" % ind,
+         "%sconst int NS = (NI + 1) | 1;   // odd: a row's columns fall in different banks" % ind]
+    ns = len(R["stage_arity"])
+    for st in range(ns):
+        L.append("%sconst int nt%d = (int)pk[1].%s;" % (ind, st, "xyzw"[st]))
+    at = "pk + 2"
+    if any(a.kind == "direct" for a in spec.args):
+        L.append("%sconst int *elems = (const int *)(%s);" % (ind, at))
+        at = "elems + ((NE + 3) & ~3)"
+    L.append("%sconst unsigned short *items = (const unsigned short *)(%s);" % (ind, at))
+    at = "(const int *)(items + ((NE * %d + 7) & ~7))" % R["ra"]
+    for st in range(ns):
+        L.append("%sconst int *tl%d = %s;" % (ind, st, at))
+        L.append("%sconst unsigned short *lx%d = (const unsigned short *)(tl%d + ((nt%d + 3) & ~3));"
+                 % (ind, st, st, st))
+        at = "(const int *)(lx%d + ((NE * %d + 7) & ~7))" % (st, R["stage_arity"][st])
+    L += ["%sconst uint2 *shorts = (const uint2 *)(%s);" % (ind, at),
+          "%sconst uint2 *longs = shorts + ((nshort + 1) & ~1);" % ind,
+          "%sconst unsigned short *ids = (const unsigned short *)(longs + ((nlong + 1) & ~1));" % ind]
+    off = "op2b_smem + 16 * room"
+    for q, (slot, st, ct, c) in enumerate(R["read_pairs"]):
+        L.append("%s%s *rd%d = (%s *)(%s);" % (ind, ct, q, ct, off))
+        off = "(unsigned char *)rd%d + ((nt%d * %d + 15) & ~15)" % (q, st, c * _CSIZE[ct])
+    for q, (ct, c, _, _) in enumerate(_rowblk_targets(spec)):
+        L.append("%s%s *S%d = (%s *)(%s);" % (ind, ct, q, ct, off))
+        off = "(unsigned char *)S%d + (((NS * %d + 1) * %d + 15) & ~15)" % (q, R["ca"], c * _CSIZE[ct])
+        # what an entry of one contribution adds second: nothing changes by it
+        zero = "(%s)-0.0" % ct if ct in ("double", "float") else "(%s)0" % ct
+        L.append("%sif (threadIdx.x < %d) S%d[NS * %d + threadIdx.x] = %s;" % (ind, c, q, R["ca"] * c, zero))
+    return L
+
+
+def _rowblk_element(spec, ind):
+    """Lines evaluating element ``i`` of the block (mesh element ``e``) into
+    the contribution arrays."""
+    R = spec.rowblk
+    RA, CA = R["ra"], R["ca"]
+    where = _rowblk_slots(spec)
+    targets = _rowblk_targets(spec)
+    parts = copy.copy(R)
+    parts["inc_pairs"] = [(j, R["map_stage"].get(m), t, c) for j, m, t, c in R["incs"]]
+    decl, pre, post, exprs, _ = _staged_element_parts(spec, parts, ind[2:], "e")
+    L, k = [], 0
+    out = []
+    for n, a in enumerate(spec.args):
+        if a.kind == "mat":
+            out.append("(%s (*)[1])&A%d" % (a.ctype, n))
+            continue
+        out.append(exprs[k])
+        k += 1
+    used = sorted({R["map_stage"][a.mslot] for a in spec.args
+                   if a.kind in ("ind", "vec", "its") and a.access == "READ"})
+    for st in used:
+        L.append("%sint sl%d[%d];" % (ind, st, R["stage_arity"][st]))
+        L.append("%s#pragma unroll" % ind)
+        L.append("%sfor (int r = 0; r < %d; ++r) sl%d[r] = lx%d[r * NE + i];" % (ind, R["stage_arity"][st], st, st))
+    L.append("%sint it[%d];" % (ind, RA))
+    L.append("%s#pragma unroll" % ind)
+    L.append("%sfor (int r = 0; r < %d; ++r) it[r] = items[r * NE + i];" % (ind, RA))
+    L += decl + pre
+    L += _itspace_open(spec, ind)
+    deep = ind + "  " * len(spec.extents)
+    for n, a in enumerate(spec.args):
+        if a.kind == "mat":
+            L.append("%s%s A%d = (%s)0;" % (deep, a.ctype, n, a.ctype))
+    L.append(_kernel_call(spec, out, deep))
+    for n, a in enumerate(spec.args):
+        if a.kind == "mat":
+            L.append("%sS%d[i1 * NS + it[i0]] = A%d;" % (deep, where[a.slot], n))
+    L += _itspace_close(spec, ind)
+    for n, a in enumerate(spec.args):
+        if a.kind == "mat" or a.access != "INC":
+            continue
+        q = where[a.slot]
+        c = targets[q][1]
+        rows = [(a.idx, "a%d" % n)] if a.kind == "ind" else [(r, "a%d[%d]" % (n, r)) for r in range(RA)]
+        for r, var in rows:
+            L.append("%sop2b_store(S%d + it[%d] * %d, %s);" % (ind, q, r, c, var))
+    return L
+
+
+def _rowblk_body(spec):
+    """Increments by the owners of the rows: a persistent grid walks the row
+    blocks (op2b_row_blocks_build).  Per block the CTA copies the block's
+    packet (cp.async, 16 bytes a time; the next one is fetched into L2
+    meanwhile), then the distinct rows read through staged Maps, to shared
+    memory; a thread evaluates whole elements, each local entry or row that
+    lands in the block's rows into the contribution arrays S ([ca][items]:
+    consecutive threads on consecutive words; what lands in another block's
+    rows goes to a column nothing reads); then the block's own rows are
+    written once, consecutive threads on consecutive CSR positions or Dat
+    values, each adding its contributions in element order to the value
+    before the loop (mz: a Mat known to be zero is not read).
+
+    The element form adds every local entry with a reduction of its own into
+    L2 (139 G/s, its bound); here rows are runs of sectors written once.
+    Measured on a B200, the loop with the memsets of its Mats: P2 K + M
+    1024 x 1024 in FP64 607 us (element form 1028), P2 512 x 512 with FP32
+    element math and compensated sums 160 us (two phases through memory 344),
+    P1 mass of 1.0 M elements 41 us (54 + 6).  What bounds it: latency of the
+    block's dependent steps at the shared memory's occupancy (packet and row
+    copies 45 %, evaluation 20 %, sums 35 % of a P1 block's cycles); blocks of
+    8 to 27 KB of contributions, a ring of packets copied two blocks ahead and
+    64 to 256 threads all measured within 5 % on P1, and smaller blocks up to
+    35 % slower on P2 (more elements evaluated twice).
+
+    ``spec.rowblk``: kind 'mat' or 'dat', ra, ca, kahan, map_stage,
+    stage_arity and read_pairs as in the staged form (READ Maps only), incs
+    [(slot, map slot, ctype, cdim)] of a Dat loop."""
+    bs, R = spec.block_size, spec.rowblk
+    targets = _rowblk_targets(spec)
+    L = []
+    L.append("extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec)))
+    _gbl_prologue(spec, L)
+    L.append("  extern __shared__ __align__(16) unsigned char op2b_smem[];")
+    L.append("  const uint4 *pk = (const uint4 *)op2b_smem;")
+    L.append("  const int room = p.col_n;   // 16-byte units of a packet")
+    L.append("  const op2b_i64 step = gridDim.x;")
+    L.append("  op2b_i64 t = blockIdx.x;")
+    L.append("  int2 td = p.rb_dir[t], tn = td;")
+    L.append("  if (t + step < p.rb_blocks) tn = p.rb_dir[t + step];")
+    L.append("  for (; t < p.rb_blocks; t += step) {")
+    L.append("    op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rb_pkt + td.x, td.y);" % bs)
+    # the directory is read two blocks ahead, so no thread waits for it
+    L.append("    td = tn;")
+    L.append("    if (t + 2 * step < p.rb_blocks) tn = p.rb_dir[t + 2 * step];")
+    L.append("    if (t + step < p.rb_blocks) op2b_rb_prefetch<%d>(p.rb_pkt + td.x, td.y);" % bs)
+    L.append("    op2b_cp_async_wait();")
+    L.append("    __syncthreads();")
+    L += _rowblk_parse(spec, "    ")
+    if R["read_pairs"]:
+        for st in range(len(R["stage_arity"])):
+            pairs = [(q, slot, ct, c) for q, (slot, s_, ct, c) in enumerate(R["read_pairs"]) if s_ == st]
+            if not pairs:
+                continue
+            L.append("    for (int r = threadIdx.x; r < nt%d; r += %d) {" % (st, bs))
+            L.append("      const op2b_i64 g = tl%d[r];" % st)
+            for q, slot, ct, c in pairs:
+                nb = c * _CSIZE[ct]
+                if nb % 4 == 0:
+                    L.append("      op2b_cp_async_srow<%d>(rd%d, r, p.d%d + g * %d);" % (nb, q, slot, c))
+                else:
+                    L.append("      for (int k = 0; k < %d; ++k) rd%d[r * %d + k] = p.d%d[g * %d + k];"
+                             % (c, q, c, slot, c))
+            L.append("    }")
+        L.append("    op2b_cp_async_wait();")
+        L.append("    __syncthreads();")
+    L.append("    for (int i = threadIdx.x; i < NE; i += %d) {" % bs)
+    if any(a.kind == "direct" for a in spec.args):
+        L.append("      const op2b_i64 e = elems[i];")
+    L += _rowblk_element(spec, "      ")
+    L.append("    }")
+    L.append("    __syncthreads();")
+    L += _rowblk_sums(spec, targets)
+    L.append("    __syncthreads();     // the next packet takes this one's place")
+    L.append("  }")
+    L.append("}")
+    return "\n".join(L)
+
+
+def _rowblk_add(R, t, v, c, s):
+    """Line adding contribution ``s`` to ``v`` (compensation ``c``)."""
+    if R["kahan"]:
+        return "{ const %s y = %s - %s, z = %s + y; %s = (z - %s) - y; %s = z; }" % (t, s, c, v, c, v, v)
+    return "%s += %s;" % (v, s)
+
+
+def _rowblk_sums(spec, targets):
+    """The block's entries: those of one or two contributions without a loop
+    over contributions (most entries of an element method's matrix), two at
+    a time per thread; then the longer ones, which would hold up their warps.
+    A Dat's row takes one thread per component."""
+    bs, R = spec.block_size, spec.rowblk
+    L = []
+    for c in sorted({c for _, c, _, _ in targets}):
+        mine = [(q, t, arr, z) for q, (t, tc, arr, z) in enumerate(targets) if tc == c]
+        comp = c > 1
+
+        def at(var):
+            return "(op2b_i64)%s * %d + m" % (var, c) if comp else var
+
+        def src(q, var):
+            return "S%d[(%s) * %d + m]" % (q, var, c) if comp else "S%d[%s]" % (q, var)
+
+        def entry(u, ind, what):
+            out = []
+            if what == "load":
+                if comp:
+                    out.append("%sconst int m = l%s %% %d;" % (ind, u, c))
+                out.append("%sconst uint2 w%s = shorts[%s];" % (ind, u, "l%s / %d" % (u, c) if comp else "l" + u))
+                for q, t, arr, z in mine:
+                    old = "%s[%s]" % (arr, at("w%s.x" % u))
+                    out.append("%s%s v%d%s = %s;" % (ind, t, q, u,
+                                                   old if z is None else "p.mz%d ? (%s)0 : %s" % (z, t, old)))
+            elif what == "add":
+                for q, t, arr, z in mine:
+                    v = "v%d%s" % (q, u)
+                    if R["kahan"]:
+                        out.append("%s{ %s c = (%s)0; %s" % (ind, t, t, _rowblk_add(
+                            R, t, v, "c", src(q, "w%s.y & 0xffffu" % u))))
+                        out.append("%s  if ((w%s.y >> 16) != none) %s }" % (ind, u, _rowblk_add(
+                            R, t, v, "c", src(q, "w%s.y >> 16" % u))))
+                    else:
+                        out.append("%s%s = (%s + %s) + %s;" % (ind, v, v, src(q, "w%s.y & 0xffffu" % u),
+                                                              src(q, "w%s.y >> 16" % u)))
+            else:
+                for q, t, arr, z in mine:
+                    out.append("%s%s[%s] = v%d%s;" % (ind, arr, at("w%s.x" % u), q, u))
+            return out
+        n = "nshort * %d" % c if comp else "nshort"
+        L.append("    {")
+        if R["kahan"]:
+            L.append("      const unsigned none = (unsigned)(NS * %d);" % R["ca"])
+        if comp:
+            L.append("      for (int l = threadIdx.x; l < %s; l += %d) {" % (n, bs))
+            for what in ("load", "add", "store"):
+                L += entry("", "        ", what)
+            L.append("      }")
+        else:
+            L.append("      int l = threadIdx.x;")
+            L.append("      for (; l + %d < %s; l += %d) {" % (bs, n, 2 * bs))
+            L.append("        const int l_a = l, l_b = l + %d;" % bs)
+            for what in ("load", "add", "store"):
+                L += entry("_a", "        ", what) + entry("_b", "        ", what)
+            L.append("      }")
+            L.append("      if (l < %s) {" % n)
+            for what in ("load", "add", "store"):
+                L += entry("", "        ", what)
+            L.append("      }")
+        L.append("      for (int l = threadIdx.x; l < %s; l += %d) {" % (n.replace("nshort", "nlong"), bs))
+        if comp:
+            L.append("        const int m = l %% %d;" % c)
+        L.append("        const uint2 w = longs[%s];" % ("l / %d" % c if comp else "l"))
+        for q, t, arr, z in mine:
+            old = "%s[%s]" % (arr, at("w.x"))
+            L.append("        %s v%d = %s%s;" % (t, q, old if z is None else "p.mz%d ? (%s)0 : %s" % (z, t, old),
+                                                ", c%d = (%s)0" % (q, t) if R["kahan"] else ""))
+        L.append("        for (unsigned k = w.y & 0xffffu; k < w.y >> 16; ++k) {")
+        L.append("          const int id = ids[k];")
+        for q, t, arr, z in mine:
+            L.append("          " + _rowblk_add(R, t, "v%d" % q, "c%d" % q, src(q, "id")))
+        L.append("        }")
+        for q, t, arr, z in mine:
+            L.append("        %s[%s] = v%d;" % (arr, at("w.x"), q))
+        L.append("      }")
+        L.append("    }")
     return L
 
 

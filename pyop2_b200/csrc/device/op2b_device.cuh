@@ -60,6 +60,19 @@ __device__ __forceinline__ void op2b_cp_async_row(void *dst, const void *src) {
 
 __device__ __forceinline__ void op2b_cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Copy of n 16-byte units to shared memory by a CTA of THREADS threads.
+template <int THREADS>
+__device__ __forceinline__ void op2b_rb_copy(uint4 *dst, const uint4 *src, int n) {
+  for (int i = threadIdx.x; i < n; i += THREADS) op2b_cp_async_row<16>(dst + i, src + i);
+}
+
+// Fetch n 16-byte units into L2.
+template <int THREADS>
+__device__ __forceinline__ void op2b_rb_prefetch(const uint4 *src, int n) {
+  for (int i = threadIdx.x * 8; i < n; i += THREADS * 8)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(src + i));
+}
+
 template <typename T, int N, bool RO>
 __device__ __forceinline__ void op2b_load(T (&dst)[N], const T *__restrict__ src) {
   constexpr int B = N * (int)sizeof(T);
