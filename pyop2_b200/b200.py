@@ -1183,13 +1183,16 @@ class RowBlocks(object):
 # aims at per incremented object (its region's elements times the bytes of one
 # element)
 _ROWBLK_THREADS = 128
-_ROWBLK_BYTES = 15360
+_ROWBLK_BYTES = 16384
 
 
-# contributions a launch adds, below which the row blocks' phases cost as much
-# as the reductions they save (P1 256 x 256, 1.2 million: 13.0 to 15.9 us by the
-# partition, 14.3 with reductions; P2 181 x 181, 2.4 million: 28.7 against 36.1)
-_ROWBLK_MIN = 3 << 19
+# contributions a launch adds, below which the form makes no difference worth
+# its tables, for local blocks below 6 x 6 and from there on.  In a graph with
+# the memsets and P1's RHS: P1 256 x 256 (1.2 million) 15.7 us against 14.4 with
+# structured numbering and 14.5 against 17.4 permuted, P1 320 x 320 (1.8 million)
+# 20.6 against 22.7; P2 128 x 128 (1.2 million) 16.5 against 22.7, 64 x 64 (0.3
+# million) 10.4 against 11.9
+_ROWBLK_MIN = (3 << 19, 1 << 20)
 
 # runs of a bound loop before its row blocks are built: the build takes what 30
 # (P2) to 80 (P1) runs then save, and the element form needs only the slot table,
@@ -1705,7 +1708,8 @@ class _BoundLoop(object):
         self._rows_later = bool(
             w is not None and nelem is None and inc_mode is None and not _partitioned(iterset)
             and (spec.mode == "lma" or (spec.mode == "atomic" and _default_mat_form()))
-            and iterset.size * w.arity * w.carity >= _ROWBLK_MIN and codegen.rowblk_capable(spec))
+            and iterset.size * w.arity * w.carity >= _ROWBLK_MIN[w.arity * w.carity >= 36]
+            and codegen.rowblk_capable(spec))
         if self._rows_later and (rows or spec.mode == "lma"):
             self._rows_later = False
             try:

@@ -1388,14 +1388,14 @@ def _rowblk_body(spec):
     The element form adds every local entry with a reduction of its own into
     L2 (139 G/s, its bound); here rows are runs of sectors written once.
     Measured on a B200, the loop with the memsets of its Mats: P2 K + M
-    1024 x 1024 in FP64 607 us (element form 1028), P2 512 x 512 with FP32
-    element math and compensated sums 160 us (two phases through memory 344),
-    P1 mass of 1.0 M elements 41 us (54 + 6).  What bounds it: latency of the
-    block's dependent steps at the shared memory's occupancy (packet and row
-    copies 45 %, evaluation 20 %, sums 35 % of a P1 block's cycles); blocks of
-    8 to 27 KB of contributions, a ring of packets copied two blocks ahead and
-    64 to 256 threads all measured within 5 % on P1, and smaller blocks up to
-    35 % slower on P2 (more elements evaluated twice).
+    1024 x 1024 in FP64 605 us (element form 1028), P2 512 x 512 with FP32
+    element math and compensated sums 143 us (two phases through memory 344),
+    P1 mass of 1.0 M elements 39 us (60).  What bounds it: shared memory
+    wavefronts (about 60 % of their rate on P2: 4 loads and 2 stores an entry,
+    72 stores an element) and the latency of a block's dependent steps at the
+    16 to 28 warps its shared memory allows.  Blocks of 8 to 20 KB of
+    contributions measured within 10 %; a ring of packets copied two blocks
+    ahead did not pay for its shared memory.
 
     ``spec.rowblk``: kind 'mat' or 'dat', ra, ca, kahan, map_stage,
     stage_arity and read_pairs as in the staged form (READ Maps only), incs

@@ -11,13 +11,14 @@
 // blocks of a hundred rows of a triangle mesh).  This file builds the tables
 // such a stub walks:
 //  * blocks: regions of elements are grown around hashed seeds by a
-//    breadth-first search through the Map, and cut by sector (which of the
-//    seed's targets an element was reached through), then level, into runs of
-//    at most `region` elements: wedges, as compact as squares and of nearly
-//    one size, which is what the shared memory of a launch is sized by; a row
-//    belongs to the block whose elements use it first.  Which region an
-//    element between two seeds joins may differ from build to build; the
-//    loop's results do not depend on it;
+//    breadth-first search through the Map and ordered by sector (which of the
+//    seed's targets an element was reached through), then level; the rows,
+//    in order of first use along that order, are cut inside each region into
+//    runs of nearly equal numbers of items ((element, map index) pairs), at
+//    most `region` elements' worth: wedges, as compact as squares and of one
+//    size, which is what the shared memory of a launch is sized by.  Which
+//    region an element between two seeds joins may differ from build to build;
+//    the loop's results do not depend on it;
 //  * one packet per block, 16-byte aligned so that a CTA copies it to shared
 //    memory while it still works on the block before:
 //      header  int32 {elements NE, short entries, long entries, items NI},
@@ -83,7 +84,7 @@ struct RbArgs {
 };
 
 // device scalars
-enum { kSFlag, kSCursor, kSMaxPacket, kSMaxTargets, kSScan = kSMaxTargets + kRbStages, kSBlocks = kSScan + 4,
+enum { kSFlag, kSCursor, kSMaxPacket, kSMaxTargets, kSScan = kSMaxTargets + kRbStages, kSBlocks = kSScan + 3,
        kSUsed, kSMaxItems, kSMaxRows, kSChanged, kSCount = kSChanged + 3 };
 
 constexpr int kRbLevels = 32;          // levels told apart in a region's order
@@ -169,28 +170,6 @@ __global__ void rb_order_kernel(int n, const int32_t *__restrict__ bucket, int32
     order[atomicAdd(&cursor[bucket[e]], 1)] = e;
 }
 
-// Runs a region is cut into.  first: the buckets' first places.
-__global__ void rb_pieces_kernel(int nregions, int buckets, int part, const int32_t *__restrict__ first,
-                                 int32_t *__restrict__ pieces) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= nregions; r += gridDim.x * blockDim.x)
-    pieces[r] = r < nregions ? (first[(int64_t)(r + 1) * buckets] - first[(int64_t)r * buckets] + part - 1) / part : 0;
-}
-
-// First element of every block, and their number.
-__global__ void rb_blocks_kernel(int nregions, int buckets, int n, const int32_t *__restrict__ first,
-                                 const int32_t *__restrict__ pieces, int32_t *__restrict__ boff,
-                                 int32_t *__restrict__ scal) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nregions; r += gridDim.x * blockDim.x) {
-    const int a = first[(int64_t)r * buckets], cnt = first[(int64_t)(r + 1) * buckets] - a;
-    const int b = pieces[r], m = pieces[r + 1] - b;
-    for (int q = 0; q < m; ++q) boff[b + q] = a + (int)((int64_t)cnt * q / m);
-    if (r == nregions - 1) {
-      boff[pieces[nregions]] = n;
-      scal[kSBlocks] = pieces[nregions];
-    }
-  }
-}
-
 // First use of every target along the elements' order (all ones: none), and
 // the number of its uses.
 __global__ void rb_first_kernel(int64_t tot, int ra, const int32_t *__restrict__ rmap,
@@ -239,19 +218,61 @@ __global__ void rb_scatter_kernel(const int32_t *__restrict__ rmap, int64_t tot,
   }
 }
 
-// First row of every block (the first uses before its first element), and the
-// largest block's items and rows.
-__global__ void rb_starts_kernel(const int32_t *__restrict__ boff, int ra, const int32_t *__restrict__ ranks,
-                                 const int32_t *__restrict__ io, int32_t *__restrict__ rstart,
+// First row of region r: the first uses before its first element (bfirst: the
+// buckets' first places).
+__device__ __forceinline__ int rb_region_row(int r, int buckets, int ra, const int32_t *bfirst,
+                                             const int32_t *ranks) {
+  return ranks[(int64_t)bfirst[(int64_t)r * buckets] * ra];
+}
+
+// Runs each region's rows are cut into, of at most `most` items as a rule.
+__global__ void rb_pieces_kernel(int nregions, int buckets, int ra, int most, const int32_t *__restrict__ bfirst,
+                                 const int32_t *__restrict__ ranks, const int32_t *__restrict__ io,
+                                 int32_t *__restrict__ pieces) {
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r <= nregions; r += gridDim.x * blockDim.x) {
+    int m = 0;
+    if (r < nregions) {
+      const int a = rb_region_row(r, buckets, ra, bfirst, ranks),
+                b = rb_region_row(r + 1, buckets, ra, bfirst, ranks);
+      m = min(b - a, (io[b] - io[a] + most - 1) / most);
+    }
+    pieces[r] = m;
+  }
+}
+
+// First row of every block, and the largest block's items and rows.
+__global__ void rb_starts_kernel(int nregions, int buckets, int ra, const int32_t *__restrict__ bfirst,
+                                 const int32_t *__restrict__ ranks, const int32_t *__restrict__ io,
+                                 const int32_t *__restrict__ pieces, int32_t *__restrict__ rstart,
                                  int32_t *__restrict__ scal) {
   int mi = 0, mr = 0;
-  const int nblocks = scal[kSBlocks];
-  for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nblocks; b += gridDim.x * blockDim.x) {
-    const int r0 = ranks[(int64_t)boff[b] * ra], r1 = ranks[(int64_t)boff[b + 1] * ra];
-    rstart[b] = r0;
-    if (b == nblocks - 1) rstart[nblocks] = r1;
-    mi = max(mi, io[r1] - io[r0]);
-    mr = max(mr, r1 - r0);
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nregions; r += gridDim.x * blockDim.x) {
+    const int a = rb_region_row(r, buckets, ra, bfirst, ranks),
+              b = rb_region_row(r + 1, buckets, ra, bfirst, ranks);
+    const int first = pieces[r], m = pieces[r + 1] - first, total = io[b] - io[a];
+    int from = a;
+    for (int q = 1; q <= m; ++q) {
+      // the first row at or past the q-th part of the items; every run has a row
+      int lo = from + 1, hi = b - (m - q);
+      if (q < m) {
+        const int want = io[a] + (int)((int64_t)total * q / m);
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (io[mid] < want) lo = mid + 1;
+          else hi = mid;
+        }
+      } else {
+        lo = b;
+      }
+      rstart[first + q - 1] = from;
+      mi = max(mi, io[lo] - io[from]);
+      mr = max(mr, lo - from);
+      from = lo;
+    }
+    if (r == nregions - 1) {
+      rstart[pieces[nregions]] = b;
+      scal[kSBlocks] = pieces[nregions];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) {
     mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, o));
@@ -557,7 +578,7 @@ int op2b_row_blocks_build(uint64_t rmap_, int32_t ra, int32_t nelem, int32_t nro
   if (nbuckets >= INT_MAX) return done(OP2B_OK, false);
   // one workspace; 64-bit keys first
   const int64_t words[] = {2LL * n, 2LL * nrows,                               // ekey, tkey
-                           n, nbuckets + 1, nbuckets + 1, n + 1, nregions + 1, most_blocks + 1,
+                           n, nbuckets + 1, nbuckets + 1, n + 1, nregions + 1,
                            nrows, nrows, tot + 1, nrows, nrows, nrows + 1, nrows + 1, tot, most_blocks + 1, kSCount};
   constexpr int kWords = sizeof words / sizeof words[0];
   int64_t at[kWords + 1] = {0};
@@ -566,17 +587,17 @@ int op2b_row_blocks_build(uint64_t rmap_, int32_t ra, int32_t nelem, int32_t nro
   uint64_t *ekey = reinterpret_cast<uint64_t *>(work);
   unsigned long long *tkey = reinterpret_cast<unsigned long long *>(work + at[1]);
   int32_t *bucket = work + at[2], *bfirst = work + at[3], *cursor = work + at[4], *eorder = work + at[5],
-          *pieces = work + at[6], *boff = work + at[7], *deg = work + at[9], *ranks = work + at[10],
-          *order = work + at[11], *rank = work + at[12], *io = work + at[13], *eo = work + at[14],
-          *list = work + at[15], *rstart = work + at[16], *scal = work + at[17];
-  unsigned *first = reinterpret_cast<unsigned *>(work + at[8]);
+          *pieces = work + at[6], *deg = work + at[8], *ranks = work + at[9], *order = work + at[10],
+          *rank = work + at[11], *io = work + at[12], *eo = work + at[13], *list = work + at[14],
+          *rstart = work + at[15], *scal = work + at[16];
+  unsigned *first = reinterpret_cast<unsigned *>(work + at[7]);
   RB_CUDA(cudaMemsetAsync(scal, 0, sizeof(int32_t) * kSCount, s));
   RB_CUDA(cudaMemsetAsync(tkey, 0xff, sizeof(uint64_t) * nrows, s));
   RB_CUDA(cudaMemsetAsync(bfirst, 0, sizeof(int32_t) * (nbuckets + 1), s));
   RB_CUDA(cudaMemsetAsync(first, 0xff, sizeof(int32_t) * nrows, s));
   RB_CUDA(cudaMemsetAsync(deg, 0, sizeof(int32_t) * nrows, s));
-  RB_CUDA(cudaMemsetAsync(io, 0, sizeof(int32_t) * (at[15] - at[13]), s));
-  // blocks of elements
+  RB_CUDA(cudaMemsetAsync(io, 0, sizeof(int32_t) * (at[14] - at[12]), s));
+  // regions of elements
   {
     int per_sm = 0, ra_ = ra, n_ = n, most = most_seeds, sb = sbits;
     RB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rb_grow_kernel, 256, 0));
@@ -591,17 +612,16 @@ int op2b_row_blocks_build(uint64_t rmap_, int32_t ra, int32_t nelem, int32_t nro
   RB_TRY(device_excl_scan(bfirst, bfirst, nbuckets + 1, scal + kSScan, s));
   RB_CUDA(cudaMemcpyAsync(cursor, bfirst, sizeof(int32_t) * nbuckets, cudaMemcpyDeviceToDevice, s));
   rb_order_kernel<<<grid(n), 256, 0, s>>>(n, bucket, cursor, eorder);
-  rb_pieces_kernel<<<grid(nregions + 1), 256, 0, s>>>(nregions, buckets, region, bfirst, pieces);
-  RB_TRY(device_excl_scan(pieces, pieces, nregions + 1, scal + kSScan, s));
-  rb_blocks_kernel<<<grid(nregions), 256, 0, s>>>(nregions, buckets, n, bfirst, pieces, boff, scal);
-  // their rows
+  // rows, and the blocks they are cut into
   rb_first_kernel<<<grid(tot), 256, 0, s>>>(tot, ra, rmap, eorder, first, deg);
   rb_flag_kernel<<<grid(tot + 1), 256, 0, s>>>(tot, ra, rmap, eorder, first, ranks);
   RB_TRY(device_excl_scan(ranks, ranks, tot + 1, scal + kSUsed, s));
   rb_rows_kernel<<<grid(tot), 256, 0, s>>>(tot, ra, rmap, eorder, ranks, deg, A.rowptr, order, rank, io, eo);
   RB_TRY(device_excl_scan(io, io, (int64_t)nrows + 1, scal + kSScan, s));
   RB_TRY(device_excl_scan(eo, eo, (int64_t)nrows + 1, scal + kSScan + 1, s));
-  rb_starts_kernel<<<grid(most_blocks), 256, 0, s>>>(boff, ra, ranks, io, rstart, scal);
+  rb_pieces_kernel<<<grid(nregions + 1), 256, 0, s>>>(nregions, buckets, ra, region * ra, bfirst, ranks, io, pieces);
+  RB_TRY(device_excl_scan(pieces, pieces, nregions + 1, scal + kSScan + 2, s));
+  rb_starts_kernel<<<grid(nregions), 256, 0, s>>>(nregions, buckets, ra, bfirst, ranks, io, pieces, rstart, scal);
   rb_scatter_kernel<<<grid(tot), 256, 0, s>>>(rmap, tot, rank, io, deg, list);
   RB_CUDA(cudaGetLastError());
   int32_t h[kSCount];
