@@ -408,32 +408,32 @@ int op2b_mat_zero_rows(uint64_t vals, uint64_t rowptr, uint64_t colidx, int32_t 
                        int32_t elem_bytes, uint64_t stream);
 
 /* ------------------------------------------------------------------------
- * Row blocks of a loop that only increments through one Map (rmap [nelem][ra],
- * nrows targets): a Dat's rows, or the entries of a scalar Mat assembled
- * through (rmap, cmap [nelem][ca]) on the CSR pattern (rowptr, colidx; both 0
- * for a Dat).  The elements are partitioned into regions of about `region`
- * elements; a block owns the rows its region's elements use first and lists
- * every element that touches them, the staged Maps' (at most 4) distinct
- * targets, and for each entry of its rows the contributions in element order
- * (pyop2/sequential.py:55-72 adds them in that order).  *rb is 0 where the
- * form does not apply: no elements, rows of too many elements for a block, or
- * an entry the pattern lacks.  Map values must lie in their target Sets.
- * Replaces the colouring and the LMA-to-CSR scatter of such a loop
- * (pyop2/plan.pyx:214-376, assets/cuda_matrix_support.jinja2:27-81).
+ * Row blocks of scalar Mat assembly through one Map pair (rmap [nelem][ra],
+ * cmap [nelem][ca]) on the CSR pattern (rowptr, colidx) of nrows rows.  The
+ * elements are grown into regions of about 3 * region elements, and the rows of
+ * a region, in order of first use, cut into blocks of about region * ra items
+ * ((element, map index) pairs).  A block lists every element that touches its
+ * rows, the staged Maps' (at most 4) distinct targets, and for each stored entry
+ * of its rows the contributions in element order (pyop2/sequential.py:55-72 adds
+ * them in that order).  *rb is 0 where the form does not apply: no elements,
+ * rows of too many elements for a block, or an entry the pattern lacks.  Map
+ * values must lie in their target Sets.  Replaces the colouring and the
+ * LMA-to-CSR scatter of such a loop (pyop2/plan.pyx:214-376,
+ * assets/cuda_matrix_support.jinja2:27-81).
  * Block b's packet starts at 16 * dir[b].start bytes of packets and takes
  * 16 * dir[b].size (dir: int32 pairs).  It holds int32 {elements NE, short
  * entries, long entries, items NI}, int32 {targets of each staged Map}, then,
  * each padded to 16 bytes: elements int32 [NE] (if ids); items uint16 [ra][NE]
  * ((element, map index) landing in the block's rows, else NI); per staged Map
  * targets int32 and indices into them uint16 [arity][NE]; short entries uint32
- * {CSR position or Dat row, contribution | second contribution << 16
+ * {CSR position, contribution | second contribution << 16
  * (ca * NS: none)}; long entries uint32 {position, first | last + 1 << 16
  * in the list}; the list uint16.  A contribution is c * NS + item, NS
  * the first odd number above NI.
  * max_targets: 4 values; max_packet in 16-byte units.
  * ---------------------------------------------------------------------- */
-int op2b_row_blocks_build(uint64_t rmap, int32_t ra, int32_t nelem, int32_t nrows, int32_t region,
-                          uint64_t cmap, int32_t ca, uint64_t rowptr, uint64_t colidx,
+int op2b_row_blocks_build(uint64_t rmap, uint64_t cmap, int32_t nelem, int32_t ra, int32_t ca,
+                          int32_t nrows, uint64_t rowptr, uint64_t colidx, int32_t region,
                           int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
                           int32_t ids, uint64_t stream, uint64_t *rb);
 int op2b_row_blocks_info(uint64_t rb, int32_t *nblocks, int32_t *max_items, int32_t *max_packet,

@@ -101,7 +101,7 @@ _SIGS = {
     "op2b_vec_dot": [u64, u64, i64, C.POINTER(C.c_double), u64],
     "op2b_cg_solve": [u64, u64, u64, i32, i64, u64, u64, i32, C.c_double, C.c_double, C.c_double,
                       i32, i32p, i32p, C.POINTER(C.c_double), u64],
-    "op2b_row_blocks_build": [u64, i32, i32, i32, i32, u64, i32, u64, u64, i32, u64p, i32p, i32,
+    "op2b_row_blocks_build": [u64, u64, i32, i32, i32, i32, u64, u64, i32, i32, u64p, i32p, i32,
                               u64, u64p],
     "op2b_row_blocks_info": [u64, i32p, i32p, i32p, i32p, u64p, u64p],
     "op2b_row_blocks_free": [u64],

@@ -1134,29 +1134,26 @@ def _incidence(m):
 
 
 class RowBlocks(object):
-    """Row blocks of a loop that increments through one Map
-    (op2b_row_blocks_build)."""
+    """Row blocks of a scalar Mat assembly (op2b_row_blocks_build)."""
 
     @classmethod
-    def of(cls, rmap, region, stage_maps, ids, sparsity=None, cmap=None):
-        """The row blocks of increments through ``rmap`` (into ``sparsity``'s
-        entries with columns ``cmap``), with the elements' ``ids`` for loops
-        that need them, built at first use and kept with the Map; None where
-        the form does not apply."""
-        tables = rmap.__dict__.setdefault("_row_block_tables", {})
-        key = (region, tuple(id(m) for m in stage_maps), ids, id(sparsity), id(cmap))
+    def of(cls, sparsity, rmap, cmap, region, stage_maps, ids):
+        """The row blocks of assembly through (rmap, cmap), with the elements'
+        ``ids`` for loops that need them, built at first use and kept with the
+        Sparsity; None where the form does not apply."""
+        tables = sparsity.__dict__.setdefault("_row_block_tables", {})
+        key = (id(rmap), id(cmap), region, tuple(id(m) for m in stage_maps), ids)
         hit = tables.get(key)
         if hit is None:
             ns = len(stage_maps)
             smap = (C.c_uint64 * max(ns, 1))(*[m._to_device().ptr for m in stage_maps])
             sar = (C.c_int32 * max(ns, 1))(*[m.dim for m in stage_maps])
             h = C.c_uint64()
-            call("op2b_row_blocks_build", rmap._to_device().ptr, rmap.dim, rmap.iterset.size,
-                 rmap.dataset.size, region, cmap._to_device().ptr if cmap is not None else 0,
-                 cmap.dim if cmap is not None else 1, sparsity._d_rowptr if sparsity else 0,
-                 sparsity._d_colidx if sparsity else 0, ns, smap, sar, int(ids), 0, C.byref(h))
-            # the Maps and the Sparsity stay alive as long as their ids are keys
-            hit = tables[key] = (cls(h.value) if h.value else None, list(stage_maps), cmap, sparsity)
+            call("op2b_row_blocks_build", rmap._to_device().ptr, cmap._to_device().ptr,
+                 rmap.iterset.size, rmap.dim, cmap.dim, rmap.dataset.size, sparsity._d_rowptr,
+                 sparsity._d_colidx, region, ns, smap, sar, int(ids), 0, C.byref(h))
+            # the Maps stay alive as long as their ids are keys
+            hit = tables[key] = (cls(h.value) if h.value else None, rmap, cmap, list(stage_maps))
         return hit[0]
 
     def __init__(self, handle):
@@ -1179,9 +1176,8 @@ class RowBlocks(object):
             pass
 
 
-# threads per CTA of the row block stubs, and bytes of contributions a block
-# aims at per incremented object (its region's elements times the bytes of one
-# element)
+# threads per CTA of the row block stubs, and bytes of contributions to one Mat
+# a block aims at (its region's elements times the bytes of one element)
 _ROWBLK_THREADS = 128
 _ROWBLK_BYTES = 16384
 
@@ -1207,37 +1203,25 @@ _runs = [0]
 def row_block_spec(spec, specs, maps, mats, kahan=False):
     """(the loop's spec in the row block form, its RowBlocks), or None where
     that form does not run the loop."""
-    kind = codegen.rowblk_capable(spec) if spec.mode in ("atomic", "lma", "staged") else None
-    if kind is None or (kind == "mat" and any(m.sparsity is not mats[0].sparsity for m in mats)):
+    if (spec.mode not in ("atomic", "lma") or not codegen.rowblk_capable(spec)
+            or any(m.sparsity is not mats[0].sparsity for m in mats) or mats[0].sparsity._dims != (1, 1)):
         return None
-    w = next(s for s in specs if s.access == "INC" and s.kind != "gbl")
+    w = next(s for s in specs if s.kind == "mat")
     reads = _region_layout([s for s in specs if s.access == "READ"], maps)
     if len(reads["stage_arity"]) > 4:
         return None
     new = copy.copy(spec)
     new.mode, new.block_size = "rowblk", _ROWBLK_THREADS
-    incs = [] if kind == "mat" else sorted({(s.slot, s.mslot, s.ctype, s.cdim) for s in specs
-                                            if s.access == "INC" and s.kind != "gbl"})
-    new.rowblk = {"kind": kind, "ra": w.arity, "ca": w.carity if kind == "mat" else 1,
-                  "kahan": bool(kahan), "map_stage": reads["map_stage"],
-                  "stage_arity": reads["stage_arity"], "read_pairs": reads["read_pairs"],
-                  "incs": incs}
+    new.rowblk = {"ra": w.arity, "ca": w.carity, "kahan": bool(kahan), "map_stage": reads["map_stage"],
+                  "stage_arity": reads["stage_arity"], "read_pairs": reads["read_pairs"]}
     new.mat_slots, new.mat_alias, new.mat_slots_rel, new.itspace_split = False, (), False, None
-    new.mat_per_entry, new.region, new.gathered = False, None, ()
-    rmap = maps[w.mslot]
-    stage_maps = [maps[k] for k in reads["stage_maps"]]
+    new.mat_per_entry, new.gathered = False, ()
     ids = any(s.kind == "direct" for s in specs)
-    # bytes one element adds to the largest contribution array
-    one = max(w.arity * new.rowblk["ca"] * c * codegen._CSIZE[t]
-              for t, c, _, _ in codegen._rowblk_targets(new))
+    # a block's contributions to the Mat of the largest entries
+    one = w.arity * w.carity * max(m.dtype.itemsize for m in mats)
     region = max(16, min(512, _ROWBLK_BYTES // one))
-    if kind == "mat":
-        sp = mats[0].sparsity
-        if sp._dims != (1, 1):
-            return None
-        rb = RowBlocks.of(rmap, region, stage_maps, ids, sp, maps[w.cmslot])
-    else:
-        rb = RowBlocks.of(rmap, region, stage_maps, ids)
+    rb = RowBlocks.of(mats[0].sparsity, maps[w.mslot], maps[w.cmslot], region,
+                      [maps[k] for k in reads["stage_maps"]], ids)
     if rb is None or codegen.rowblk_smem(new, rb.max_items, rb.max_packet, rb.max_targets) > \
             _state['smem_optin']:
         return None

@@ -1216,76 +1216,41 @@ def _atomic_element(spec, ind, ranges=None):
 
 
 def rowblk_capable(spec):
-    """Loops the row block form can run: every write is an INC, all of them
-    through one Map -- scalar Mats over their full local tensor (rows on i0,
-    columns on i1, one (row, column) Map pair) or Dats at every index of the
-    Map, each (Dat, index) once -- every other argument is READ, and at most
-    four Maps are read through.  Returns 'mat', 'dat' or None."""
+    """Loops the row block form can run: every write is an INC into a scalar
+    Mat over its full local tensor (rows on i0, columns on i1), each Mat once,
+    all through one (row, column) Map pair; every other argument is READ."""
     mats = [a for a in spec.args if a.kind == "mat"]
-    incs = [a for a in spec.args if a.kind != "mat" and a.access != "READ"]
-    if any(a.access != "INC" or a.kind not in ("ind", "vec", "its") for a in incs):
-        return None
-    if any(a.ctype not in _CSIZE for a in mats + incs):
-        return None
-    if mats:
-        ok = (not incs and len(spec.extents) == 2 and len({a.slot for a in mats}) == len(mats)
-              and all(a.access == "INC" and a.rm * a.cm == 1 and (a.idx, a.cidx) == (0, 1)
-                      and (a.mslot, a.cmslot) == (mats[0].mslot, mats[0].cmslot)
-                      and tuple(spec.extents) == (a.arity, a.carity) for a in mats))
-        return "mat" if ok else None
-    if not incs or len({a.mslot for a in incs}) != 1:
-        return None
-    seen = {}
-    for a in incs:
-        if a.kind == "its" and (len(spec.extents) != 1 or a.idx != 0 or a.ext != a.arity):
-            return None
-        at = [a.idx] if a.kind == "ind" else list(range(a.arity))
-        got = seen.setdefault(a.slot, [])
-        if set(got) & set(at):
-            return None
-        got += at
-    if any(sorted(got) != list(range(incs[0].arity)) for got in seen.values()):
-        return None
-    # an INC Dat read in the same loop would see other blocks' sums
-    if any(a.access == "READ" and a.kind != "gbl" and a.slot in seen for a in spec.args):
-        return None
-    return "dat"
+    return (bool(mats) and len(spec.extents) == 2 and len({a.slot for a in mats}) == len(mats)
+            and all(a.kind == "mat" or a.access == "READ" for a in spec.args)
+            and all(a.access == "INC" and a.rm * a.cm == 1 and (a.idx, a.cidx) == (0, 1)
+                    and (a.mslot, a.cmslot) == (mats[0].mslot, mats[0].cmslot)
+                    and tuple(spec.extents) == (a.arity, a.carity) and a.ctype in _CSIZE for a in mats))
 
 
-def _rowblk_targets(spec):
-    """(ctype, cdim, name of the device array, index of the zero flag or None)
-    per incremented Mat or Dat slot."""
-    if spec.rowblk["kind"] == "mat":
-        return [(spec.mats[j], 1, "p.mv%d" % j, j) for j in range(len(spec.mats))]
-    out = {}
-    for a in spec.args:
-        if a.access == "INC":
-            out[a.slot] = (a.ctype, a.cdim, "p.d%d" % a.slot, None)
-    return [out[j] for j in sorted(out)]
-
-
-def _rowblk_slots(spec):
-    """Mat or Dat slot -> its place in _rowblk_targets."""
-    if spec.rowblk["kind"] == "mat":
-        return {j: j for j in range(len(spec.mats))}
-    return {j: q for q, j in enumerate(sorted({a.slot for a in spec.args if a.access == "INC"}))}
+def _rowblk_sum_decl(spec):
+    """(declaration, bytes) of the struct of one contribution to every Mat of
+    the loop: one shared-memory access for all of them (two doubles: 16
+    bytes)."""
+    sizes = [_CSIZE[t] for t in spec.mats]
+    align = max(sizes)
+    if len(set(sizes)) == 1 and len(sizes) == 2:
+        align = min(16, sum(sizes))
+    at = 0
+    for s in sizes:
+        at = (at + s - 1) // s * s + s
+    return ("struct __align__(%d) op2b_rb_sum { %s };" % (
+        align, " ".join("%s v%d;" % (t, j) for j, t in enumerate(spec.mats))), (at + align - 1) // align * align)
 
 
 def rowblk_smem(spec, max_items, max_packet, max_targets):
     """Dynamic shared memory of a row block launch: a packet, the staged READ
-    rows, and per incremented object the contributions of a block, [ca][odd
-    number of items], and one place of zeros."""
+    rows, and the contributions of a block, [ca][odd number of items], with
+    one place of zeros."""
     R = spec.rowblk
-    nb = 16 * max_packet + rowblk_rows(spec, max_targets)
-    for ctype, cdim, _, _ in _rowblk_targets(spec):
-        nb += ((((max_items + 1) | 1) * R["ca"] + 1) * cdim * _CSIZE[ctype] + 15) // 16 * 16
-    return nb
-
-
-def rowblk_rows(spec, max_targets):
-    """Bytes of the staged READ rows of a block."""
-    return sum((max_targets[st] * cdim * _CSIZE[ctype] + 15) // 16 * 16
-               for slot, st, ctype, cdim in spec.rowblk["read_pairs"])
+    nb = 16 * max_packet
+    for slot, st, ctype, cdim in R["read_pairs"]:
+        nb += (max_targets[st] * cdim * _CSIZE[ctype] + 15) // 16 * 16
+    return nb + (((max_items + 1) | 1) * R["ca"] + 1) * _rowblk_sum_decl(spec)[1]
 
 
 def _rowblk_parse(spec, ind):
@@ -1314,61 +1279,38 @@ def _rowblk_parse(spec, ind):
     for q, (slot, st, ct, c) in enumerate(R["read_pairs"]):
         L.append("%s%s *rd%d = (%s *)(%s);" % (ind, ct, q, ct, off))
         off = "(unsigned char *)rd%d + ((nt%d * %d + 15) & ~15)" % (q, st, c * _CSIZE[ct])
-    for q, (ct, c, _, _) in enumerate(_rowblk_targets(spec)):
-        L.append("%s%s *S%d = (%s *)(%s);" % (ind, ct, q, ct, off))
-        off = "(unsigned char *)S%d + (((NS * %d + 1) * %d + 15) & ~15)" % (q, R["ca"], c * _CSIZE[ct])
-        # what an entry of one contribution adds second: nothing changes by it
-        zero = "(%s)-0.0" % ct if ct in ("double", "float") else "(%s)0" % ct
-        L.append("%sif (threadIdx.x < %d) S%d[NS * %d + threadIdx.x] = %s;" % (ind, c, q, R["ca"] * c, zero))
+    L.append("%sop2b_rb_sum *S = (op2b_rb_sum *)(%s);" % (ind, off))
+    # what an entry of one contribution adds second: nothing changes by it
+    L.append("%sif (threadIdx.x == 0) S[NS * %d] = {%s};" % (ind, R["ca"], ", ".join(
+        "(%s)-0.0" % t if t in ("double", "float") else "(%s)0" % t for t in spec.mats)))
     return L
 
 
 def _rowblk_element(spec, ind):
     """Lines evaluating element ``i`` of the block (mesh element ``e``) into
-    the contribution arrays."""
+    the contributions."""
     R = spec.rowblk
-    RA, CA = R["ra"], R["ca"]
-    where = _rowblk_slots(spec)
-    targets = _rowblk_targets(spec)
-    parts = copy.copy(R)
-    parts["inc_pairs"] = [(j, R["map_stage"].get(m), t, c) for j, m, t, c in R["incs"]]
+    parts = dict(R, inc_pairs=[])
     decl, pre, post, exprs, _ = _staged_element_parts(spec, parts, ind[2:], "e")
-    L, k = [], 0
-    out = []
-    for n, a in enumerate(spec.args):
-        if a.kind == "mat":
-            out.append("(%s (*)[1])&A%d" % (a.ctype, n))
-            continue
-        out.append(exprs[k])
-        k += 1
-    used = sorted({R["map_stage"][a.mslot] for a in spec.args
-                   if a.kind in ("ind", "vec", "its") and a.access == "READ"})
-    for st in used:
-        L.append("%sint sl%d[%d];" % (ind, st, R["stage_arity"][st]))
+    exprs = iter(exprs)
+    args = ["(%s (*)[1])&A%d" % (a.ctype, n) if a.kind == "mat" else next(exprs)
+            for n, a in enumerate(spec.args)]
+    mats = {a.slot: n for n, a in enumerate(spec.args) if a.kind == "mat"}
+    L = []
+    for st, ar in enumerate(R["stage_arity"]):
+        L.append("%sint sl%d[%d];" % (ind, st, ar))
         L.append("%s#pragma unroll" % ind)
-        L.append("%sfor (int r = 0; r < %d; ++r) sl%d[r] = lx%d[r * NE + i];" % (ind, R["stage_arity"][st], st, st))
-    L.append("%sint it[%d];" % (ind, RA))
+        L.append("%sfor (int r = 0; r < %d; ++r) sl%d[r] = lx%d[r * NE + i];" % (ind, ar, st, st))
+    L.append("%sint it[%d];" % (ind, R["ra"]))
     L.append("%s#pragma unroll" % ind)
-    L.append("%sfor (int r = 0; r < %d; ++r) it[r] = items[r * NE + i];" % (ind, RA))
+    L.append("%sfor (int r = 0; r < %d; ++r) it[r] = items[r * NE + i];" % (ind, R["ra"]))
     L += decl + pre
     L += _itspace_open(spec, ind)
     deep = ind + "  " * len(spec.extents)
-    for n, a in enumerate(spec.args):
-        if a.kind == "mat":
-            L.append("%s%s A%d = (%s)0;" % (deep, a.ctype, n, a.ctype))
-    L.append(_kernel_call(spec, out, deep))
-    for n, a in enumerate(spec.args):
-        if a.kind == "mat":
-            L.append("%sS%d[i1 * NS + it[i0]] = A%d;" % (deep, where[a.slot], n))
+    L += ["%s%s A%d = (%s)0;" % (deep, spec.mats[j], n, spec.mats[j]) for j, n in sorted(mats.items())]
+    L.append(_kernel_call(spec, args, deep))
+    L.append("%sS[i1 * NS + it[i0]] = {%s};" % (deep, ", ".join("A%d" % n for _, n in sorted(mats.items()))))
     L += _itspace_close(spec, ind)
-    for n, a in enumerate(spec.args):
-        if a.kind == "mat" or a.access != "INC":
-            continue
-        q = where[a.slot]
-        c = targets[q][1]
-        rows = [(a.idx, "a%d" % n)] if a.kind == "ind" else [(r, "a%d[%d]" % (n, r)) for r in range(RA)]
-        for r, var in rows:
-            L.append("%sop2b_store(S%d + it[%d] * %d, %s);" % (ind, q, r, c, var))
     return L
 
 
@@ -1377,13 +1319,13 @@ def _rowblk_body(spec):
     blocks (op2b_row_blocks_build).  Per block the CTA copies the block's
     packet (cp.async, 16 bytes a time; the next one is fetched into L2
     meanwhile), then the distinct rows read through staged Maps, to shared
-    memory; a thread evaluates whole elements, each local entry or row that
-    lands in the block's rows into the contribution arrays S ([ca][items]:
-    consecutive threads on consecutive words; what lands in another block's
-    rows goes to a column nothing reads); then the block's own rows are
-    written once, consecutive threads on consecutive CSR positions or Dat
-    values, each adding its contributions in element order to the value
-    before the loop (mz: a Mat known to be zero is not read).
+    memory; a thread evaluates whole elements, each local entry that lands in
+    the block's rows into the contributions S ([ca][items]: consecutive threads
+    on consecutive places; what lands in another block's rows goes to a column
+    nothing reads); then the block's own entries are written once, consecutive
+    threads on consecutive CSR positions, each adding its contributions in
+    element order to the value before the loop (mz: a Mat known to be zero is
+    not read).
 
     The element form adds every local entry with a reduction of its own into
     L2 (139 G/s, its bound); here rows are runs of sectors written once.
@@ -1397,12 +1339,10 @@ def _rowblk_body(spec):
     contributions measured within 10 %; a ring of packets copied two blocks
     ahead did not pay for its shared memory.
 
-    ``spec.rowblk``: kind 'mat' or 'dat', ra, ca, kahan, map_stage,
-    stage_arity and read_pairs as in the staged form (READ Maps only), incs
-    [(slot, map slot, ctype, cdim)] of a Dat loop."""
+    ``spec.rowblk``: ra, ca, kahan, and map_stage, stage_arity and read_pairs
+    as in the staged form."""
     bs, R = spec.block_size, spec.rowblk
-    targets = _rowblk_targets(spec)
-    L = []
+    L = [_rowblk_sum_decl(spec)[0]]
     L.append("extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec)))
     _gbl_prologue(spec, L)
     L.append("  extern __shared__ __align__(16) unsigned char op2b_smem[];")
@@ -1444,99 +1384,66 @@ def _rowblk_body(spec):
     L += _rowblk_element(spec, "      ")
     L.append("    }")
     L.append("    __syncthreads();")
-    L += _rowblk_sums(spec, targets)
+    L += _rowblk_sums(spec)
     L.append("    __syncthreads();     // the next packet takes this one's place")
     L.append("  }")
     L.append("}")
     return "\n".join(L)
 
 
-def _rowblk_add(R, t, v, c, s):
-    """Line adding contribution ``s`` to ``v`` (compensation ``c``)."""
-    if R["kahan"]:
-        return "{ const %s y = %s - %s, z = %s + y; %s = (z - %s) - y; %s = z; }" % (t, s, c, v, c, v, v)
-    return "%s += %s;" % (v, s)
-
-
-def _rowblk_sums(spec, targets):
+def _rowblk_sums(spec):
     """The block's entries: those of one or two contributions without a loop
     over contributions (most entries of an element method's matrix), two at
-    a time per thread; then the longer ones, which would hold up their warps.
-    A Dat's row takes one thread per component."""
+    a time per thread; then the longer ones, which would hold up their warps."""
     bs, R = spec.block_size, spec.rowblk
-    L = []
-    for c in sorted({c for _, c, _, _ in targets}):
-        mine = [(q, t, arr, z) for q, (t, tc, arr, z) in enumerate(targets) if tc == c]
-        comp = c > 1
+    kahan = R["kahan"]
+    mats = list(enumerate(spec.mats))
 
-        def at(var):
-            return "(op2b_i64)%s * %d + m" % (var, c) if comp else var
+    def add(j, t, v, c, s):
+        if kahan:
+            return "{ const %s y = %s - %s, z = %s + y; %s = (z - %s) - y; %s = z; }" % (t, s, c, v, c, v, v)
+        return "%s += %s;" % (v, s)
 
-        def src(q, var):
-            return "S%d[(%s) * %d + m]" % (q, var, c) if comp else "S%d[%s]" % (q, var)
+    def load(u, ind):
+        return ["%sconst uint2 w%s = shorts[l%s];" % (ind, u, u)] + [
+            "%s%s v%d%s = p.mz%d ? (%s)0 : p.mv%d[w%s.x];" % (ind, t, j, u, j, t, j, u) for j, t in mats]
 
-        def entry(u, ind, what):
-            out = []
-            if what == "load":
-                if comp:
-                    out.append("%sconst int m = l%s %% %d;" % (ind, u, c))
-                out.append("%sconst uint2 w%s = shorts[%s];" % (ind, u, "l%s / %d" % (u, c) if comp else "l" + u))
-                for q, t, arr, z in mine:
-                    old = "%s[%s]" % (arr, at("w%s.x" % u))
-                    out.append("%s%s v%d%s = %s;" % (ind, t, q, u,
-                                                   old if z is None else "p.mz%d ? (%s)0 : %s" % (z, t, old)))
-            elif what == "add":
-                for q, t, arr, z in mine:
-                    v = "v%d%s" % (q, u)
-                    if R["kahan"]:
-                        out.append("%s{ %s c = (%s)0; %s" % (ind, t, t, _rowblk_add(
-                            R, t, v, "c", src(q, "w%s.y & 0xffffu" % u))))
-                        out.append("%s  if ((w%s.y >> 16) != none) %s }" % (ind, u, _rowblk_add(
-                            R, t, v, "c", src(q, "w%s.y >> 16" % u))))
-                    else:
-                        out.append("%s%s = (%s + %s) + %s;" % (ind, v, v, src(q, "w%s.y & 0xffffu" % u),
-                                                              src(q, "w%s.y >> 16" % u)))
-            else:
-                for q, t, arr, z in mine:
-                    out.append("%s%s[%s] = v%d%s;" % (ind, arr, at("w%s.x" % u), q, u))
-            return out
-        n = "nshort * %d" % c if comp else "nshort"
-        L.append("    {")
-        if R["kahan"]:
-            L.append("      const unsigned none = (unsigned)(NS * %d);" % R["ca"])
-        if comp:
-            L.append("      for (int l = threadIdx.x; l < %s; l += %d) {" % (n, bs))
-            for what in ("load", "add", "store"):
-                L += entry("", "        ", what)
-            L.append("      }")
-        else:
-            L.append("      int l = threadIdx.x;")
-            L.append("      for (; l + %d < %s; l += %d) {" % (bs, n, 2 * bs))
-            L.append("        const int l_a = l, l_b = l + %d;" % bs)
-            for what in ("load", "add", "store"):
-                L += entry("_a", "        ", what) + entry("_b", "        ", what)
-            L.append("      }")
-            L.append("      if (l < %s) {" % n)
-            for what in ("load", "add", "store"):
-                L += entry("", "        ", what)
-            L.append("      }")
-        L.append("      for (int l = threadIdx.x; l < %s; l += %d) {" % (n.replace("nshort", "nlong"), bs))
-        if comp:
-            L.append("        const int m = l %% %d;" % c)
-        L.append("        const uint2 w = longs[%s];" % ("l / %d" % c if comp else "l"))
-        for q, t, arr, z in mine:
-            old = "%s[%s]" % (arr, at("w.x"))
-            L.append("        %s v%d = %s%s;" % (t, q, old if z is None else "p.mz%d ? (%s)0 : %s" % (z, t, old),
-                                                ", c%d = (%s)0" % (q, t) if R["kahan"] else ""))
-        L.append("        for (unsigned k = w.y & 0xffffu; k < w.y >> 16; ++k) {")
-        L.append("          const int id = ids[k];")
-        for q, t, arr, z in mine:
-            L.append("          " + _rowblk_add(R, t, "v%d" % q, "c%d" % q, src(q, "id")))
-        L.append("        }")
-        for q, t, arr, z in mine:
-            L.append("        %s[%s] = v%d;" % (arr, at("w.x"), q))
-        L.append("      }")
-        L.append("    }")
+    def sums(u, ind):
+        L = ["%sconst op2b_rb_sum s%s = S[w%s.y & 0xffffu];" % (ind, u, u)]
+        if not kahan:
+            L.append("%sconst op2b_rb_sum t%s = S[w%s.y >> 16];" % (ind, u, u))
+            return L + ["%sv%d%s = (v%d%s + s%s.v%d) + t%s.v%d;" % (ind, j, u, j, u, u, j, u, j) for j, t in mats]
+        L += ["%s%s c%d%s = (%s)0; %s" % (ind, t, j, u, t, add(j, t, "v%d%s" % (j, u), "c%d%s" % (j, u),
+                                                             "s%s.v%d" % (u, j))) for j, t in mats]
+        L.append("%sif ((w%s.y >> 16) != (unsigned)(NS * %d)) {" % (ind, u, R["ca"]))
+        L.append("%s  const op2b_rb_sum t%s = S[w%s.y >> 16];" % (ind, u, u))
+        L += ["%s  %s" % (ind, add(j, t, "v%d%s" % (j, u), "c%d%s" % (j, u), "t%s.v%d" % (u, j)))
+              for j, t in mats]
+        return L + ["%s}" % ind]
+
+    def store(u, ind):
+        return ["%sp.mv%d[w%s.x] = v%d%s;" % (ind, j, u, j, u) for j, t in mats]
+    L = ["    {",
+         "      int l = threadIdx.x;",
+         "      for (; l + %d < nshort; l += %d) {" % (bs, 2 * bs),
+         "        const int l_a = l, l_b = l + %d;" % bs]
+    for part in (load, sums, store):
+        L += part("_a", "        ") + part("_b", "        ")
+    L += ["      }", "      if (l < nshort) {"]
+    for part in (load, sums, store):
+        L += part("", "        ")
+    L += ["      }",
+          "      for (int l = threadIdx.x; l < nlong; l += %d) {" % bs,
+          "        const uint2 w = longs[l];"]
+    for j, t in mats:
+        L.append("        %s v%d = p.mz%d ? (%s)0 : p.mv%d[w.x]%s;" % (
+            t, j, j, t, j, ", c%d = (%s)0" % (j, t) if kahan else ""))
+    L += ["        for (unsigned k = w.y & 0xffffu; k < w.y >> 16; ++k) {",
+          "          const op2b_rb_sum s = S[ids[k]];"]
+    L += ["          " + add(j, t, "v%d" % j, "c%d" % j, "s.v%d" % j) for j, t in mats]
+    L.append("        }")
+    L += ["        p.mv%d[w.x] = v%d;" % (j, j) for j, t in mats]
+    L += ["      }", "    }"]
     return L
 
 

@@ -1,9 +1,9 @@
-// Row blocks: indirect increments run by the owners of the incremented rows.
+// Row blocks: Mat assembly run by the owners of the rows.
 //
-// A loop whose only writes are increments through one Map (a Dat's rows, or a
-// scalar Mat's entries in those rows) can be run by row instead of by element:
-// a CTA owns a block of rows, evaluates every element that touches one of
-// them into shared memory, and writes each of its rows once, adding the row's
+// A loop whose only writes are increments of scalar Mats through one (row Map,
+// column Map) pair can be run by row instead of by element: a CTA owns a block
+// of rows, evaluates every element that touches one of them into shared memory,
+// and writes every stored entry of its rows once, adding the entry's
 // contributions in element order (the order of pyop2/sequential.py:55-72).
 // No add is atomic, there are no colours, and the result does not depend on
 // scheduling; the price is that an element whose rows belong to several
@@ -31,11 +31,11 @@
 //      per staged Map (the loop reads Dats through it): targets int32 [nt],
 //              the block's distinct targets in order of first use, and
 //              lidx uint16 [arity][NE], each element's targets in that list
-//      shorts  per entry of one or two contributions, rows in order and a
-//              Mat's columns in order: {where it goes (Mat: CSR position, Dat:
-//              row), first contribution | second << 16}; an entry of one has
-//              ca * NS as its second, a place the stub fills with -0.0
-//      longs   per other entry: {where it goes, first | last + 1 << 16 of its
+//      shorts  per entry of one or two contributions, rows in order, columns
+//              in order: {CSR position, first contribution | second << 16}; an
+//              entry of one has ca * NS as its second, a place the stub fills
+//              with -0.0
+//      longs   per other entry: {CSR position, first | last + 1 << 16 of its
 //              contributions in list} (apart: a warp waits for its longest)
 //      list    uint16: the long entries' contributions
 //    A contribution is its place in the block's shared array [ca][NS], NS the
@@ -203,7 +203,7 @@ __global__ void rb_rows_kernel(int64_t tot, int ra, const int32_t *__restrict__ 
     order[i] = t;
     rank[t] = i;
     io[i] = deg[t];
-    eo[i] = rowptr ? rowptr[t + 1] - rowptr[t] : 1;
+    eo[i] = rowptr[t + 1] - rowptr[t];
   }
 }
 
@@ -351,10 +351,7 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
   for (int i = tid; i <= nr; i += kRbThreads) {
     ro[i] = A.io[row0 + i] - i0;
     re[i] = A.eo[row0 + i] - e0;
-    if (i < nr) {
-      const int t = A.order[row0 + i];
-      rb[i] = A.rowptr ? A.rowptr[t] : t;
-    }
+    if (i < nr) rb[i] = A.rowptr[A.order[row0 + i]];
   }
   __syncthreads();
   // row of item / entry k: the last row whose offset is <= k
@@ -406,13 +403,10 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
   // contributions of entry j of row rl; the elements' columns take the hash
   // arrays' place
   int *cols = tab;                          // [NE][ca]
-  if (A.rowptr) {
-    for (int k = tid; k < NE * ca; k += kRbThreads) cols[k] = A.cmap[(int64_t)elems[k / ca] * ca + k % ca];
-    __syncthreads();
-  }
+  for (int k = tid; k < NE * ca; k += kRbThreads) cols[k] = A.cmap[(int64_t)elems[k / ca] * ca + k % ca];
+  __syncthreads();
   auto entry_col = [&](int j, int rl) { return A.colidx[rb[rl] + j - re[rl]]; };
   auto count_of = [&](int j, int rl) {
-    if (!A.rowptr) return ro[rl + 1] - ro[rl];
     const int col = entry_col(j, rl);
     int cnt = 0;
     for (int i = ro[rl]; i < ro[rl + 1]; ++i) {
@@ -481,8 +475,8 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
     int ia = ic + block_excl_scan(cnt > kRbShort ? cnt : 0, &idt);
     if (cnt > 0) {
       found += cnt;
-      const unsigned pos = (unsigned)(rb[rl] + (A.rowptr ? j - re[rl] : 0));
-      const int col = A.rowptr ? entry_col(j, rl) : 0;
+      const unsigned pos = (unsigned)(rb[rl] + j - re[rl]);
+      const int col = entry_col(j, rl);
       unsigned two[kRbShort] = {0u, (unsigned)(ca * ns)};
       if (cnt > kRbShort) longs[la] = make_uint2(pos, (unsigned)ia | (unsigned)(ia + cnt) << 16);
       int k = 0;
@@ -490,7 +484,7 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
         const int e = it[i] / ra, r = it[i] - e * ra;
         const int *c = cols + eloc[i] * ca;
         for (int q = 0; q < ca; ++q)
-          if (!A.rowptr || c[q] == col) {
+          if (c[q] == col) {
             const unsigned id = (unsigned)(q * ns + own[r * NE + eloc[i]]);
             if (cnt > kRbShort) ids[ia + k] = (unsigned short)id;
             else two[k] = id;
@@ -524,18 +518,16 @@ static void rowblk_release(RowBlocks *p, cudaStream_t s) {
 
 extern "C" {
 
-int op2b_row_blocks_build(uint64_t rmap_, int32_t ra, int32_t nelem, int32_t nrows, int32_t region,
-                          uint64_t cmap_, int32_t ca, uint64_t rowptr_, uint64_t colidx_,
+int op2b_row_blocks_build(uint64_t rmap_, uint64_t cmap_, int32_t nelem, int32_t ra, int32_t ca,
+                          int32_t nrows, uint64_t rowptr_, uint64_t colidx_, int32_t region,
                           int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
                           int32_t ids, uint64_t stream, uint64_t *out) {
   OP2B_REQUIRE_INIT();
-  const bool mat = rowptr_ != 0;
-  if (nelem < 0 || ra <= 0 || nrows < 0 || region <= 0 || nstage < 0 || !out || (nelem > 0 && !rmap_) ||
-      (mat && (ca <= 0 || (nelem > 0 && (!cmap_ || !colidx_)))) || (nstage > 0 && (!stage_map || !stage_arity)))
+  if (nelem < 0 || ra <= 0 || ca <= 0 || nrows < 0 || region <= 0 || nstage < 0 || !out ||
+      (nelem > 0 && (!rmap_ || !cmap_ || !rowptr_ || !colidx_)) || (nstage > 0 && (!stage_map || !stage_arity)))
     return set_error(OP2B_ERR_ARG, "row blocks: nelem %d arity %d/%d rows %d region %d", nelem, ra, ca, nrows,
                      region);
   *out = 0;
-  if (!mat) ca = 1;
   const int64_t tot = (int64_t)nelem * ra;
   if (tot == 0 || nrows == 0 || tot * ca >= INT_MAX || nstage > kRbStages) return OP2B_OK;
   cudaStream_t s = stream_of(stream);
@@ -628,7 +620,7 @@ int op2b_row_blocks_build(uint64_t rmap_, int32_t ra, int32_t nelem, int32_t nro
   RB_CUDA(cudaMemcpyAsync(h, scal, sizeof h, cudaMemcpyDeviceToHost, s));
   RB_CUDA(cudaStreamSynchronize(s));
   const int nblocks = h[kSBlocks];
-  const int64_t mi = h[kSMaxItems], keys = mi * std::max(mat ? (ca + 1) / 2 : 1, *std::max_element(A.st.arity, A.st.arity + kRbStages));
+  const int64_t mi = h[kSMaxItems], keys = mi * std::max((ca + 1) / 2, *std::max_element(A.st.arity, A.st.arity + kRbStages));
   // rows of too many elements for a block: the caller keeps its other form
   if (mi * ca > kRbMaxContrib || keys > kRbMaxKeys || mi * A.st.rows > 2 * kRbMaxKeys ||
       h[kSMaxRows] > 8192)
