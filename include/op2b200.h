@@ -71,6 +71,9 @@ int op2b_memcpy_h2d_small(uint64_t dst, const void *src, uint64_t bytes, uint64_
 /* Device-to-host copy that returns at once (stream-ordered; complete when an
  * event recorded after it completes).  dst must be pinned host memory
  * (op2b_host_alloc) for the copy to be asynchronous. */
+/* Host copies of n arrays (dst[i], src[i]: host addresses, no overlap) by up to
+ * eight threads, for results of megabytes into fresh memory. */
+int op2b_host_copy(int32_t n, const uint64_t *dst, const uint64_t *src, const uint64_t *bytes);
 int op2b_memcpy_d2h_async(void *dst, uint64_t src, uint64_t bytes, uint64_t stream);
 int op2b_memcpy_d2d(uint64_t dst, uint64_t src, uint64_t bytes, uint64_t stream);
 int op2b_memset(uint64_t dst, int value, uint64_t bytes, uint64_t stream);
@@ -158,7 +161,15 @@ int op2b_function_occupancy(uint64_t fn, uint32_t block, uint32_t smem, int32_t 
  * The generated stubs all take a single struct argument. */
 int op2b_launch(uint64_t fn, uint32_t grid, uint32_t block, uint32_t smem,
                 uint64_t stream, const void *params, uint64_t nbytes);
-/* on != 0: op2b_launch and op2b_launch_colored launch with programmatic
+/* The same on the library's stream from a record the caller keeps: one
+ * argument to convert per launch instead of seven. */
+typedef struct op2b_launch_desc {
+  uint64_t fn;
+  const void *params;
+  uint32_t grid, block, smem, reserved;
+} op2b_launch_desc;
+int op2b_launch_record(const op2b_launch_desc *d);
+/* on != 0: op2b_launch, op2b_launch_record and op2b_launch_colored launch with programmatic
  * stream serialisation, so a stub's CTAs may be scheduled while the kernel
  * before it on the stream finishes; the generated stubs wait for that
  * kernel's completion (griddepcontrol.wait) before touching memory, so

@@ -31,6 +31,7 @@ _SIGS = {
     "op2b_host_free": [u64],
     "op2b_memcpy_h2d": [u64, P, u64, u64],
     "op2b_memcpy_d2h": [P, u64, u64, u64],
+    "op2b_host_copy": [i32, u64p, u64p, u64p],
     "op2b_memcpy_d2h_async": [P, u64, u64, u64],
     "op2b_memcpy_h2d_small": [u64, P, u64, u64],
     "op2b_memcpy_d2d": [u64, u64, u64, u64],
@@ -69,6 +70,7 @@ _SIGS = {
     "op2b_module_global": [u64, charp, u64p, u64p],
     "op2b_function_set_smem": [u64, i32],
     "op2b_function_occupancy": [u64, u32, u32, i32p],
+    "op2b_launch_record": [P],
     "op2b_launch": [u64, u32, u32, u32, u64, P, u64],
     "op2b_set_programmatic_launch": [i32],
     "op2b_launch_colored": [u64, i32, i32p, u32, u32, u64, P, u64, u64],

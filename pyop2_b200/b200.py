@@ -169,6 +169,26 @@ def pinned_empty(shape, dtype):
     return arr_holder.array
 
 
+def copies(arrays):
+    """Fresh copies of a dict of numpy arrays.  Most of such a copy is the page
+    faults of the new memory, which several threads take at once
+    (op2b_host_copy); a thread that waits in it does not hold the interpreter."""
+    out, dst, src, nbytes = {}, [], [], []
+    for k, v in arrays.items():
+        if type(v) is not np.ndarray or v.dtype.hasobject or not v.flags.c_contiguous:
+            out[k] = np.array(v)
+            continue
+        out[k] = a = np.empty(v.shape, v.dtype)
+        dst.append(a.ctypes.data)
+        src.append(v.ctypes.data)
+        nbytes.append(v.nbytes)
+    n = len(dst)
+    if n:
+        u64s = C.c_uint64 * n
+        call("op2b_host_copy", n, u64s(*dst), u64s(*src), u64s(*nbytes))
+    return out
+
+
 class _PinnedHolder(object):
     def __init__(self, array, raw):
         self.array = array
@@ -1956,6 +1976,10 @@ class _BoundLoop(object):
             # the header's second colour field: room of a packet
             struct.pack_into("<i", self._buf, codegen.ParamLayout.COL_OFFSET + 4,
                              self.row_blocks.max_packet)
+        # op2b_launch_desc of the launches over the whole set
+        self._desc = C.create_string_buffer(struct.pack("<QQIIII", self.module.fn, C.addressof(self._buf),
+                                                        self.grid, self.block_size, self.launch_smem, 0))
+        self._desc_ptr = C.addressof(self._desc)
 
     def run(self, loop, rng=None):
         """Run the loop over its whole set, or over elements [start, end)
@@ -2056,8 +2080,7 @@ class _BoundLoop(object):
             finally:
                 struct.pack_into("<qq", buf, 16, 0, self.range_end)
         else:
-            call("op2b_launch", mod.fn, self.grid, self.block_size, self.launch_smem, 0, params,
-                 self.layout.nbytes)
+            call("op2b_launch_record", self._desc_ptr)
         if self.spec.mode == "lma":
             kahan = 1 if self.kahan else 0            # OP2B_LMA_KAHAN
             for buf, inc, target, cdim, ntargets, arity, mask in self.lma:
@@ -2075,7 +2098,8 @@ class _BoundLoop(object):
         for d in self._written:
             d._state = DEVICE
             d._wgen += 1
-            maybe_setflags(d._data, write=False)
+            if d._data.flags.writeable:      # unlike setflags, cheap to ask
+                maybe_setflags(d._data, write=False)
         for k in self._reducing:
             args[self._gbl[k][1]].data._state = DEVICE
         for m in self.mats:

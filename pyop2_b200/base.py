@@ -436,6 +436,11 @@ class Dat(DataCarrier):
 
     def __call__(self, path, access):
         if access is READ or access is INC or access is WRITE or access is RW:
+            # the common case first: a Map element (Map.__getitem__'s Arg)
+            if type(path) is Arg:
+                path._dat = self
+                path._access = access
+                return path
             return self._arg(path, access)
         return self._call_checked(path, access)
 
@@ -658,8 +663,13 @@ class Global(DataCarrier):
         self._name = name or "global_%d" % Global._globalcount
         Global._globalcount += 1
 
-    @validate_in(('access', _modes, ModeValueError))
     def __call__(self, access):
+        if access is READ or access is INC or access is MIN or access is MAX:
+            return _new_arg(self, None, None, access)
+        return self._call_checked(access)
+
+    @validate_in(('access', _modes, ModeValueError))
+    def _call_checked(self, access):
         return _new_arg(self, None, None, access)
 
     def __str__(self):

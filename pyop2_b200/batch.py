@@ -35,7 +35,8 @@ from .exceptions import DeviceError
 TILE_DTYPE = np.dtype([("seg", "<i4"), ("pad", "<i4"), ("first", "<i8")])
 
 # (loop signature, block size, elements per thread, min blocks) ->
-# (module, BatchLayout, has finalisation, finalisation function, CTAs per SM)
+# (spec, module, BatchLayout, has finalisation, finalisation function, CTAs per
+# SM without shared memory)
 _COMPILED = {}
 
 
@@ -145,6 +146,7 @@ class LoopInstance(object):
             raise ValueError("batched form %r (atomic or color)" % form)
         self.spec = spec
         self.key = spec.key()
+        self.layout = codegen.ParamLayout(spec)
         self.iterset = info['iterset']
         specs = info['specs']
         written = {id(a.data) for a, s in zip(loop.args, specs)
@@ -167,7 +169,7 @@ class LoopInstance(object):
                              nthrcol=d["nthrcol"], thrcol=d["thrcol"], ind_map=d["ind_map"],
                              ind_sizes=d["ind_sizes"], ind_offs=d["ind_offs"],
                              loc_map=d["loc_map"])
-        self.params = codegen.ParamLayout(self.spec).pack(self.size, 0, self.size, self.vals)
+        self.params = self.layout.pack(self.size, 0, self.size, self.vals)
 
     def recast(self, form, part_size=256):
         """The same loop over the same objects in another batched form."""
@@ -184,7 +186,7 @@ class LoopInstance(object):
         new = object.__new__(LoopInstance)
         new.form, new.plan = self.form, None
         new._loop_args = None
-        new.spec, new.key = self.spec, self.key
+        new.spec, new.key, new.layout = self.spec, self.key, self.layout
         by_id = {id(k): v for k, v in subs.items()}   # Maps compare by structure
         r = lambda o: by_id.get(id(o), o)  # noqa: E731
         new.iterset = r(self.iterset)
@@ -213,7 +215,7 @@ class LoopInstance(object):
         the objects in ``ptrs`` (object -> device address) read and write the
         given addresses instead: raw device memory of the same layout (e.g.
         a request's arena).  Maps, Sparsity and sizes are shared."""
-        layout = codegen.ParamLayout(self.spec)
+        layout = self.layout
         buf = bytearray(self.params)
         by_id = {id(k): v for k, v in ptrs.items()}
         hit = 0
@@ -284,13 +286,25 @@ class BatchLoop(object):
             if inst.key != key:
                 raise ValueError("instance %d of the batch has a different loop signature" % n)
         self._mats = list({id(m): m for i in self.instances for m in i.mats}.values())
-        spec = copy.copy(self.instances[0].spec)
-        spec.block_size = int(block_size or cfg.cfg['block_size'])
-        spec.batch = int(elems_per_thread)
-        spec.min_blocks = int(min_blocks)
-        if spec.batch < 1:
+        block_size, batch = int(block_size or cfg.cfg['block_size']), int(elems_per_thread)
+        min_blocks = int(min_blocks)
+        if batch < 1:
             raise ValueError("elems_per_thread must be >= 1")
-        self.spec = spec
+        # an engine makes several batches a step: everything but the segments and
+        # tiles is looked up
+        ckey = (key, block_size, batch, min_blocks)
+        hit = _COMPILED.get(ckey)
+        if hit is None:
+            spec = copy.copy(self.instances[0].spec)
+            spec.block_size, spec.batch, spec.min_blocks = block_size, batch, min_blocks
+            module = b200._get_module(spec)
+            layout = codegen.BatchLayout(spec)
+            has_fin = len(layout.fields) > 5
+            fin = module.function(codegen.batch_stub_names(spec)[1]) if has_fin else 0
+            hit = _COMPILED[ckey] = (spec, module, layout, has_fin, fin,
+                                     module.occupancy(module.fn, block_size, 0))
+        self.spec, self.module, self.layout, self.has_fin, self.fin, occ = hit
+        spec = self.spec
         self.form = self.instances[0].form
         self.config = dict(block_size=spec.block_size, elems_per_thread=spec.batch,
                            min_blocks=spec.min_blocks, ctas_per_sm=int(ctas_per_sm))
@@ -299,19 +313,11 @@ class BatchLoop(object):
                                block_size=spec.block_size, min_blocks=spec.min_blocks,
                                ctas_per_sm=int(ctas_per_sm))
         self.smem = max((i.plan.nshared for i in self.instances if i.plan is not None), default=0)
-        ckey = (key, spec.block_size, spec.batch, spec.min_blocks)
-        hit = _COMPILED.get(ckey)
-        if hit is None:
-            module = b200._get_module(spec)
-            layout = codegen.BatchLayout(spec)
-            has_fin = len(layout.fields) > 5
-            fin = module.function(codegen.batch_stub_names(spec)[1]) if has_fin else 0
-            hit = _COMPILED[ckey] = (module, layout, has_fin, fin)
-        self.module, self.layout, self.has_fin, self.fin = hit
         if self.smem > b200._state['smem_optin']:
             raise DeviceError("coloured batch needs %d bytes of shared memory per block" % self.smem)
         self.module.ensure_smem(self.smem)
-        occ = self.module.occupancy(self.module.fn, spec.block_size, self.smem)
+        if self.smem:
+            occ = self.module.occupancy(self.module.fn, spec.block_size, self.smem)
         if self.form == "color":
             self._init_colored(occ, int(ctas_per_sm))
             return

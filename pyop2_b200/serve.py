@@ -355,7 +355,7 @@ class ChainJob(Job):
 
 def keep_results(job, views):
     """Default consumer: keep a copy of the results on the job."""
-    job.result = {k: np.array(v) for k, v in views.items()}
+    job.result = b200.copies(views)
 
 
 # ------------------------------------------------------------------- engine

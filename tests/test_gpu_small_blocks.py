@@ -1,0 +1,51 @@
+"""Device blocks of Globals: the slab of small blocks and its ends."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def op2(backend):
+    from pyop2_b200 import op2
+    return op2
+
+
+@pytest.mark.parametrize("nbytes", [1, 16, 248, 256, 264])
+def test_small_blocks_do_not_overlap(op2, nbytes):
+    """More blocks at once than the slab holds, each with its own bytes; what is
+    released is handed out again."""
+    from pyop2_b200.b200 import DeviceBuffer
+    n = 300
+    for turn in range(2):
+        bufs = [DeviceBuffer(nbytes) for _ in range(n)]
+        ptrs = sorted(b.ptr for b in bufs)
+        assert all(b - a >= max(nbytes, 16) for a, b in zip(ptrs, ptrs[1:]))
+        want = [np.full(nbytes, (7 * k + turn) % 251, np.uint8) for k in range(n)]
+        for b, w in zip(bufs, want):
+            b.from_host(w)
+        for b, w in zip(bufs, want):
+            got = np.empty(nbytes, np.uint8)
+            b.to_host(got)
+            np.testing.assert_array_equal(got, w)
+        if turn == 0:
+            first = set(ptrs)
+            del bufs[::2], b
+    assert first & set(ptrs)
+
+
+def test_fresh_globals_of_a_repeated_reduction(op2):
+    """A new Global per loop call, several alive at once: each its own sum."""
+    s = op2.Set(1000, 1, "s")
+    d = op2.Dat(s, np.arange(1000.0), np.float64, "d")
+    k = op2.Kernel("void add(double *x, double *g) { *g += *x; }", "add")
+    kept = []
+    for n in range(12):
+        g = op2.Global(1, float(n), np.float64, "g")
+        op2.par_loop(k, s, d(op2.IdentityMap, op2.READ), g(op2.INC))
+        if n % 3 == 0:
+            kept.append((n, g))
+        else:
+            assert g.data[0] == n + 499500.0
+    assert [g.data[0] for _, g in kept] == [n + 499500.0 for n, _ in kept]
