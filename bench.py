@@ -493,7 +493,7 @@ def run_gpu(args, ws, rank, local):
         b200.synchronize()
         t0 = time.perf_counter()
         b200.RegionPlan(rp.set_size, rp.part_size, rp.region_size, rp._keep[0], rp._keep[1:],
-                        rp.stage_inc)
+                        rp.stage_inc, even=rp.even)
         b200.synchronize()
         partition_ms = round((time.perf_counter() - t0) * 1e3, 3)
     res_bytes = bytes_["res_calc"]

@@ -258,6 +258,24 @@ int op2b_region_plan_info(uint64_t plan, int32_t *nblocks, int32_t *nregions, in
  * element at position pos is tlist[toff[b*nstage+s] + loc[(row0(s)+r)*set_size+pos]],
  * 6 thrcol [set_size] (thread colour per position), 7 nthrcol [nblocks]. */
 int op2b_region_plan_array(uint64_t plan, int32_t which, uint64_t *dptr, int64_t *count);
+/* The same with the elements' order cut into runs of exactly part_size, whatever
+ * regions they lie in: every block (but the last) fills its CTA.  Within a block
+ * the elements of one row-0 target of grow_map lie next to each other. */
+int op2b_region_plan_build_even(int32_t set_size, int32_t part_size, int32_t region_size,
+                                uint64_t grow_map, int32_t grow_arity, int32_t grow_ntargets,
+                                int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
+                                const int32_t *stage_inc, uint64_t stream, uint64_t *plan);
+/* One packet per block for the summing staged form (at most 4 staged Maps), built
+ * at the first call.  Block b's packet starts at 16 * dir[b].x bytes and has
+ * dir[b].y units of 16: uint32 {NE, 0, 0, 0}, {targets of staged Maps 0..3}; with
+ * ids the elements int32 [NE]; per staged Map the targets int32 [nt] and, uint16
+ * [arity][NE], the indices of each row's targets; where stage_inc[s] != 0, uint16
+ * too, the end of each target's run [nt] and the runs [arity * NE]: contribution
+ * row * NE + element, ascending.  Each part is padded to a unit.  No reference
+ * counterpart (its kernels add colour by colour,
+ * assets/cuda_indirect_loop.jinja2). */
+int op2b_region_plan_packets(uint64_t plan, const int32_t *stage_inc, int32_t ids, uint64_t stream,
+                             uint64_t *dir, uint64_t *packets, int32_t *max_elems, int32_t *max_packet);
 /* Renumber a built plan's staged slots so that the rows eight consecutive
  * positions of a block read (one quarter-warp of a staged stub, for any CTA
  * size) lie in distinct 16-byte shared-memory bank groups where the targets

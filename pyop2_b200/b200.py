@@ -882,17 +882,18 @@ class RegionPlan(object):
     ``region_size`` elements), cut into blocks of at most ``part_size``
     elements, with each block's distinct targets of every staged Map and
     thread colours over the targets of the staged Maps flagged in
-    ``stage_inc``."""
+    ``stage_inc``.  ``even``: the order cut into runs of exactly ``part_size``,
+    whatever their regions (op2b_region_plan_build_even)."""
 
     def __init__(self, set_size, part_size, region_size, grow_map, stage_maps, stage_inc=None,
-                 bank_slots=False):
+                 bank_slots=False, even=False):
         ns = len(stage_maps)
         smap = (C.c_uint64 * max(ns, 1))(*[m._to_device().ptr for m in stage_maps])
         sar = (C.c_int32 * max(ns, 1))(*[m.dim for m in stage_maps])
         sinc = (C.c_int32 * max(ns, 1))(*[1 if (stage_inc is None or f) else 0
                                           for f in (stage_inc or [1] * ns)])
         h = C.c_uint64()
-        call("op2b_region_plan_build", set_size, part_size, region_size, grow_map._to_device().ptr,
+        call("op2b_region_plan_build_even" if even else "op2b_region_plan_build", set_size, part_size, region_size, grow_map._to_device().ptr,
              grow_map.dim, grow_map.dataset.total_size, ns, smap, sar, sinc, 0, C.byref(h))
         self._handle = h.value
         if bank_slots:
@@ -906,13 +907,23 @@ class RegionPlan(object):
         self.max_nthrcol = mt.value
         self.max_count = list(mc)[:ns]
         self.set_size, self.part_size, self.nstage = set_size, part_size, ns
-        self.region_size, self.stage_inc = region_size, stage_inc
+        self.region_size, self.stage_inc, self.even = region_size, stage_inc, bool(even)
         self._keep = [grow_map] + list(stage_maps)
         self.dptr, self.counts = {}, {}
         for k, name in enumerate(_REGION_ARRAYS):
             p, n = C.c_uint64(), C.c_int64()
             call("op2b_region_plan_array", self._handle, k, C.byref(p), C.byref(n))
             self.dptr[name], self.counts[name] = p.value, n.value
+
+    def packets(self, inc_stages, ids):
+        """(directory pointer, packet pointer, most elements of a block, most
+        16-byte units of a packet) of the summing staged form."""
+        ns = self.nstage
+        inc = (C.c_int32 * max(ns, 1))(*[int(st in inc_stages) for st in range(ns)])
+        d, p, me, mp = C.c_uint64(), C.c_uint64(), C.c_int32(), C.c_int32()
+        call("op2b_region_plan_packets", self._handle, inc, int(ids), 0, C.byref(d), C.byref(p),
+             C.byref(me), C.byref(mp))
+        return d.value, p.value, me.value, mp.value
 
     def host_array(self, name):
         out = np.zeros(self.counts[name], dtype=np.int16 if name == "loc" else np.int32)
@@ -1069,15 +1080,19 @@ def region_plan(iterset, maps, region, size=None):
     ``size`` elements, default all)."""
     n = iterset.size if size is None else int(size)
     ps = region["part_size"]
-    rs = int(cfg.cfg['region_size']) or max(1, ps // 2)
+    rs = int(cfg.cfg['region_size']) or max(1, 5 * ps // 4 if region.get("sums") else ps // 2)
     reps = [maps[k] for k in region["stage_maps"]]
     grow = reps[region["grow"]]
-    inc = [st in region["inc_stages"] for st in range(len(reps))]
+    # thread colours over the INC Maps' targets (none in the summing form, whose
+    # positions stay in the order of the search)
+    sums = bool(region.get("sums"))
+    inc = [st in region["inc_stages"] and not sums for st in range(len(reps))]
     banks = bool(cfg.cfg['staged_bank_slots'])
-    key = (n, ps, rs, id(grow), tuple(id(m) for m in reps), tuple(inc), banks)
+    key = (n, ps, rs, id(grow), tuple(id(m) for m in reps), tuple(inc), banks,
+           (tuple(region["inc_stages"]), region["ids"]) if sums else None)
     plan = _REGION_CACHE.get(key)
     if plan is None:
-        plan = _REGION_CACHE[key] = RegionPlan(n, ps, rs, grow, reps, inc, banks)
+        plan = _REGION_CACHE[key] = RegionPlan(n, ps, rs, grow, reps, inc, banks, even=sums)
     return plan
 
 
@@ -1548,7 +1563,14 @@ def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=Non
             spec.block_size = bs = int(cfg.cfg['staged_block_size'])
         # blocks of at most part_size elements; the stub runs ept passes of bs
         ps = int(cfg.cfg['partition_size']) or 384
-        R["part_size"] = ps = max(1, min(ps, 16384 // max(R["stage_arity"])))
+        ps = max(1, min(ps, 16384 // max(R["stage_arity"])))
+        if (int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
+                and not cfg.cfg['staged_tl_regs']):
+            part = codegen.staged_sums(spec, min(ps, int(cfg.cfg['partition_size'])))
+            if part:
+                R["sums"], ps = True, part
+                R["ids"] = any(s.kind == "direct" for s in specs)
+        R["part_size"] = ps
         R["ept"] = (ps + bs - 1) // bs
         if int(cfg.cfg['staged_pair']) == 2:
             R["pair"] = 2
@@ -1704,6 +1726,7 @@ class _BoundLoop(object):
         iterset = info['iterset']
         args = loop.args
         self.row_blocks = None
+        self.room = 0       # 16-byte units of a packet (row blocks, summing staged form)
         self._runs, self._last_run = 0, -_ROWBLK_RECENT
         # Mat assembly by the owners of the rows (see codegen._rowblk_body): at
         # once in place of the two-phase form, whose own tables cost as much to
@@ -1837,15 +1860,24 @@ class _BoundLoop(object):
             self.region_plan = rp
             for name in _REGION_ARRAYS:
                 vals["rg_" + name] = rp.dptr[name]
-            self.launch_smem = codegen.staged_smem(spec, rp.max_count)
+            sums = ()
+            if spec.region.get("sums"):
+                vals["rg_dir"], vals["rg_pkt"], *sums = rp.packets(spec.region["inc_stages"],
+                                                                   spec.region["ids"])
+                vals["rg_blocks"], self.room = rp.nblocks, sums[1]
+            self.launch_smem = codegen.staged_smem(spec, rp.max_count, *sums)
             if self.launch_smem > _state['smem_optin']:
                 raise _StagedTooLarge()
             self.module.ensure_smem(self.launch_smem)
             self.grid = rp.nblocks
-            self.max_grid = max(1, rp.nblocks)
+            if sums:
+                occ = max(1, self.module.occupancy(self.module.fn, spec.block_size, self.launch_smem))
+                self.grid = min(rp.nblocks, occ * _state['sm_count'])
+            self.max_grid = max(1, self.grid)
         elif spec.mode == "rowblk":
             rb = self.row_blocks
             vals.update(rb.vals)
+            self.room = rb.max_packet
             self.launch_smem = codegen.rowblk_smem(spec, rb.max_items, rb.max_packet, rb.max_targets)
             self.module.ensure_smem(self.launch_smem)
             occ = max(1, self.module.occupancy(self.module.fn, bs, self.launch_smem))
@@ -1972,10 +2004,9 @@ class _BoundLoop(object):
         n = self.nelem
         self._buf = C.create_string_buffer(self.layout.pack(n, 0, self.range_end, vals),
                                            self.layout.nbytes)
-        if self.row_blocks is not None:
+        if self.room:
             # the header's second colour field: room of a packet
-            struct.pack_into("<i", self._buf, codegen.ParamLayout.COL_OFFSET + 4,
-                             self.row_blocks.max_packet)
+            struct.pack_into("<i", self._buf, codegen.ParamLayout.COL_OFFSET + 4, self.room)
         # op2b_launch_desc of the launches over the whole set
         self._desc = C.create_string_buffer(struct.pack("<QQIIII", self.module.fn, C.addressof(self._buf),
                                                         self.grid, self.block_size, self.launch_smem, 0))

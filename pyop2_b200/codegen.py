@@ -165,6 +165,8 @@ class ParamLayout(object):
         if spec.mode == "staged":
             f += ["rg_order", "rg_boff", "rg_tlist", "rg_toff", "rg_tcnt", "rg_loc", "rg_thrcol",
                   "rg_nthrcol"]
+            if spec.region.get("sums"):
+                f += ["rg_dir", "rg_pkt", "rg_blocks"]
         if spec.mode == "rowblk":
             f += ["rb_dir", "rb_pkt", "rb_blocks"]
             f += ["mz%d" % j for j in range(len(spec.mats))]
@@ -214,6 +216,7 @@ def _struct_decl(spec, layout):
              "rg_order": "const int *", "rg_boff": "const int *", "rg_tlist": "const int *",
              "rg_toff": "const int *", "rg_tcnt": "const int *", "rg_loc": "const short *",
              "rg_thrcol": "const int *", "rg_nthrcol": "const int *",
+             "rg_dir": "const int2 *", "rg_pkt": "const uint4 *", "rg_blocks": "op2b_i64 ",
              "rb_dir": "const int2 *", "rb_pkt": "const uint4 *", "rb_blocks": "op2b_i64 "}
     for n in layout.fields:
         if n in types:
@@ -743,15 +746,57 @@ _CSIZE = {"double": 8, "float": 4, "int": 4, "unsigned int": 4, "long": 8, "long
           "char": 1, "unsigned char": 1, "signed char": 1}
 
 
-def staged_smem(spec, max_count):
-    """Dynamic shared memory of a staged launch: the staged READ rows and
-    the INC accumulators, each 16-byte aligned, at the largest per-block
-    target counts."""
+def staged_smem(spec, max_count, max_elems=0, max_packet=0):
+    """Dynamic shared memory of a staged launch at the largest per-block
+    counts, each array 16-byte aligned: the staged READ rows and the INC
+    accumulators, or with ``sums`` the contributions of ``max_elems`` elements
+    and two packets of ``max_packet`` 16-byte units."""
     R = spec.region
-    nb = 0
-    for (slot, st, ctype, cdim) in R["read_pairs"] + R["inc_pairs"]:
+    nb = 32 * max_packet
+    for (slot, st, ctype, cdim) in R["read_pairs"]:
         nb += (max_count[st] * cdim * _CSIZE[ctype] + 15) // 16 * 16
+    for (slot, st, ctype, cdim) in R["inc_pairs"]:
+        rows = max_elems * R["stage_arity"][st] if R.get("sums") else max_count[st]
+        nb += (rows * cdim * _CSIZE[ctype] + 15) // 16 * 16
     return nb
+
+
+# Elements of a block of the summing staged form: 256 while their contributions
+# take 24 KB, else 128, up to 96 KB.  Measured over 0.84 million triangles, INC rows
+# of c doubles through a of their nodes (colour form / 256 / 128 elements,
+# us): a = 2: c = 2 14.8 / 12.7, c = 4 21.4 / 17.8, c = 8 36.0 / 33.9 / 31.1,
+# c = 16 85 / 89 / 68, c = 32 388 / 396 / 313; a = 3: c = 1 16.2 / 13.0,
+# c = 4 31.2 / 23.4, c = 8 54.5 / 46.2 / 41.2, c = 24 330 / 276 / 217; beyond,
+# the contributions of 128 elements leave one CTA on an SM.
+_SUMS_PARTS = ((256, 24 << 10), (128, 96 << 10))
+
+
+def staged_sums(spec, part_size=0):
+    """Elements per block with which a staged loop stores its contributions and
+    sums them per target (``part_size`` if given), or 0 where it adds them colour
+    by colour: every INC (Dat, staged Map) pair has to be incremented through each
+    row of the Map once, and a block's contributions to fit."""
+    R = spec.region
+    rows = {}
+    for a in spec.args:
+        if a.kind in ("ind", "vec", "its") and a.access == "INC":
+            st = R["map_stage"][a.mslot]
+            rows.setdefault((a.slot, st), []).extend(
+                [a.idx] if a.kind == "ind" else range(a.arity if a.kind == "vec" else a.ext))
+    if (len(R["stage_arity"]) > 4 or part_size > 1024
+            or any(sorted(r) != list(range(R["stage_arity"][st])) for (_, st), r in rows.items())):
+        return 0
+    one = sum(R["stage_arity"][st] * c * _CSIZE[t] for _, st, t, c in R["inc_pairs"])
+    if part_size:
+        return part_size if part_size * one <= _SUMS_PARTS[-1][1] else 0
+    return next((n for n, room in _SUMS_PARTS if n * one <= room), 0)
+
+
+def _sums_chunk(ctype, cdim):
+    """(values per shared-memory access, accesses per row) of a contribution."""
+    size = _CSIZE[ctype]
+    chunk = next((b for b in (16, 8, 4) if b >= size and cdim * size % b == 0), size)
+    return chunk // size, cdim * size // chunk
 
 
 def staged_used(spec):
@@ -792,6 +837,19 @@ def _staged_copy_rows(R, used, bs, ind, dst, n, tl):
     L = []
     for st in used:
         pairs = [(q, slot, t, c) for q, (slot, s_, t, c) in enumerate(R["read_pairs"]) if s_ == st]
+        # rows of several 16-byte chunks: one chunk per thread, so that a warp's
+        # copy names half or a quarter as many cache lines
+        for q, slot, t, c in [w for w in pairs if w[3] * _CSIZE[w[2]] in (32, 64, 128)]:
+            nb = c * _CSIZE[t]
+            L.append("%sfor (int u = threadIdx.x; u < %s * %d; u += %d) {" % (ind, n % st, nb // 16, bs))
+            L.append("%s  const int r = u / %d;" % (ind, nb // 16))
+            L.append("%s  const op2b_i64 g = %s[r];" % (ind, tl % st))
+            if R.get("padded"):
+                L.append("%s  if (g < 0) continue;   // padding slot" % ind)
+            L.append("%s  op2b_cp_async_schunk<%d>(%s, r, u %% %d, p.d%d + g * %d);"
+                     % (ind, nb, dst % q, nb // 16, slot, c))
+            L.append("%s}" % ind)
+        pairs = [w for w in pairs if w[3] * _CSIZE[w[2]] not in (32, 64, 128)]
         if not pairs:
             continue
         L.append("%sfor (int r = threadIdx.x; r < %s; r += %d) {" % (ind, n % st, bs))
@@ -1028,6 +1086,160 @@ def _staged_passes(spec, R, used, bs, ind):
     return L
 
 
+def _sums_parse(spec, ind):
+    """Lines naming the parts of the packet at pk, the staged rows and the
+    contributions."""
+    R = spec.region
+    ns = len(R["stage_arity"])
+    L = ["%sconst int NE = (int)pk->x;" % ind]
+    for st in range(ns):
+        L.append("%sconst int n_s%d = (int)pk[1].%s;" % (ind, st, "xyzw"[st]))
+    at = "pk + 2"
+    if R["ids"]:
+        L.append("%sconst int *elems = (const int *)(%s);" % (ind, at))
+        at = "elems + ((NE + 3) & ~3)"
+    for st in range(ns):
+        L.append("%sconst int *tl_s%d = (const int *)(%s);" % (ind, st, at))
+        L.append("%sconst unsigned short *lx%d = (const unsigned short *)(tl_s%d + ((n_s%d + 3) & ~3));"
+                 % (ind, st, st, st))
+        at = "lx%d + ((NE * %d + 7) & ~7)" % (st, R["stage_arity"][st])
+        if st in R["inc_stages"]:
+            L.append("%sconst unsigned short *end%d = %s, *list%d = end%d + ((n_s%d + 7) & ~7);"
+                     % (ind, st, at, st, st, st))
+            at = "list%d + ((NE * %d + 7) & ~7)" % (st, R["stage_arity"][st])
+    off = "op2b_smem + 32 * room"
+    for q, (slot, st, t, c) in enumerate(R["read_pairs"]):
+        L.append("%s%s *rd%d = (%s *)(%s);" % (ind, t, q, t, off))
+        off = "(unsigned char *)rd%d + ((n_s%d * %d + 15) & ~15)" % (q, st, c * _CSIZE[t])
+    for q, (slot, st, t, c) in enumerate(R["inc_pairs"]):
+        L.append("%s%s *S%d = (%s *)(%s);" % (ind, t, q, t, off))
+        off = "(unsigned char *)S%d + ((NE * %d + 15) & ~15)" % (q, R["stage_arity"][st] * c * _CSIZE[t])
+    return L
+
+
+def _sums_element(spec, ind):
+    """Lines evaluating element ``i`` of the block, each contribution to a place
+    of its own (row * NE + i of the contributions, laid out as staged rows)."""
+    R = spec.region
+    decl, pre, post, exprs, adds = _staged_element(spec, R, ind[2:])
+    L = []
+    for st in staged_used(spec):
+        ar = R["stage_arity"][st]
+        L.append("%sint sl%d[%d];" % (ind, st, ar))
+        L.append("%s#pragma unroll" % ind)
+        L.append("%sfor (int r = 0; r < %d; ++r) sl%d[r] = lx%d[r * NE + i];" % (ind, ar, st, st))
+    L += decl + pre
+    L += _itspace_open(spec, ind)
+    L.append(_kernel_call(spec, exprs, ind + "  " * len(spec.extents)))
+    L += _itspace_close(spec, ind)
+    L += post
+    for var, lrow, q, c in adds:
+        L.append("%sop2b_srow_store(S%d, %s * NE + i, %s);" % (ind, q, lrow[lrow.index("[") + 1:-1], var))
+    return L
+
+
+def _sums_flush(spec, ind):
+    """One thread per piece of a target's row adds the target's contributions;
+    the sums are added to the Dat by whole rows."""
+    R, bs = spec.region, spec.block_size
+    L = []
+    for q, (slot, st, t, c) in enumerate(R["inc_pairs"]):
+        ve, k = _sums_chunk(t, c)
+        rows = c > 1 and 32 % c == 0      # rows added by neighbouring lanes: whole warps
+        L.append("%sfor (int u0 = threadIdx.x & ~31; u0 < n_s%d * %d; u0 += %d) {" % (ind, st, k, bs))
+        L.append("%s  const int u = u0 + (threadIdx.x & 31), r = u / %d, m = u - r * %d;" % (ind, k, k))
+        L.append("%s  int g = 0;" % ind)
+        L.append("%s  %s s[%d] = {%s};" % (ind, t, ve, ", ".join(["(%s)0" % t] * ve)))
+        L.append("%s  if (r < n_s%d) {" % (ind, st))
+        L.append("%s    g = tl_s%d[r];" % (ind, st))
+        L.append("%s    const int last = end%d[r];" % (ind, st))
+        L.append("%s    for (int l = r ? end%d[r - 1] : 0; l < last; ++l) {" % (ind, st))
+        L.append("%s      const int id = list%d[l];" % (ind, st))
+        L.append("%s      const sum%d x = *(const sum%d *)((const char *)S%d + id * %d + op2b_srow_layout<%d>::"
+                 "chunk(id, m) * %d);" % (ind, q, q, q, c * _CSIZE[t], c * _CSIZE[t], ve * _CSIZE[t]))
+        L.append("%s      %s" % (ind, " ".join("s[%d] += x.v[%d];" % (v, v) for v in range(ve))))
+        L.append("%s    }" % ind)
+        if not rows:
+            for v in range(ve):
+                L.append("%s    op2b_atomic_add(p.d%d + (op2b_i64)g * %d + m * %d + %d, s[%d]);" % (
+                    ind, slot, c, ve, v, v))
+        L.append("%s  }" % ind)
+        if rows:
+            L.append("%s  #pragma unroll" % ind)
+            L.append("%s  for (int i = 0; i < %d; ++i) {" % (ind, ve))
+            L.append("%s    int row, c; op2b_i64 to;" % ind)
+            L.append("%s    const %s x = op2b_row_share<%d, %d>(i, s, g, row, c, to);" % (ind, t, k, ve))
+            L.append("%s    if (u0 / %d + row < n_s%d) op2b_atomic_add(p.d%d + to * %d + c, x);"
+                     % (ind, k, st, slot, c))
+            L.append("%s  }" % ind)
+        L.append("%s}" % ind)
+    return L
+
+
+def _sums_body(spec):
+    """The staged form without colours: a persistent grid walks the blocks of an
+    evenly cut partition.  A block's packet (op2b_region_plan_packets) is copied
+    to shared memory while the block before it runs, so that of the chain of
+    directory, target ids and target rows only the rows are waited for.  Each
+    element's contributions are stored to places of their own, and the packet's
+    lists say which ones a target's thread adds: no colour rounds with their
+    barriers, no accumulators to read and write per element, and the elements of
+    one target next to each other, so that neighbouring lanes read the same staged
+    rows.
+
+    Measured on a B200, replayed alone: airfoil 1200 x 600 res_calc 53.6 us with
+    colours, 43.9 here; P1's right-hand side over 1.0 M triangles 23.0 us, 17.9
+    here; the whole airfoil step 199 us, 177 here.  What bounds it: shared memory wavefronts (74 % of
+    their rate while it runs: one per row a copy gathers, and the conflicts of
+    reading staged rows by index); issue slots 52 %.  Blocks of 64 to 320 elements
+    and 64 to 256 threads measured within 8 %; cutting the order evenly fills the
+    CTAs that blocks of whole regions left 40 % empty."""
+    bs, R = spec.block_size, spec.region
+    L = []
+    for q, (slot, st, t, c) in enumerate(R["inc_pairs"]):
+        ve = _sums_chunk(t, c)[0]
+        L.append("struct __align__(%d) sum%d { %s v[%d]; };" % (ve * _CSIZE[t], q, t, ve))
+    L.append("extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec)))
+    _gbl_prologue(spec, L)
+    L += ["  extern __shared__ __align__(16) unsigned char op2b_smem[];",
+          "  const int room = p.col_n;   // 16-byte units of a packet",
+          "  const op2b_i64 step = gridDim.x;",
+          "  op2b_i64 t = blockIdx.x;",
+          "  int2 tn = p.rg_dir[t];",
+          "  op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rg_pkt + tn.x, tn.y);" % bs,
+          "  if (t + step < p.rg_blocks) tn = p.rg_dir[t + step];",
+          "  for (int odd = 0; t < p.rg_blocks; t += step, odd ^= 1) {",
+          "    op2b_cp_async_wait();",
+          "    __syncthreads();         // the packet is here, and the block before is done",
+          "    const uint4 *pk = (const uint4 *)op2b_smem + odd * room;"]
+    # the packet is parsed again after each barrier: cheaper than to keep its parts
+    # in registers while the kernel runs
+    L.append("    {")
+    L += _sums_parse(spec, "      ")
+    L += _staged_copy_rows(R, staged_used(spec), bs, "      ", "rd%d", "n_s%d", "tl_s%d")
+    L += ["    }",
+          "    op2b_cp_async_commit();",
+          "    if (t + step < p.rg_blocks) op2b_rb_copy<%d>((uint4 *)op2b_smem + (odd ^ 1) * room, "
+          "p.rg_pkt + tn.x, tn.y);" % bs,
+          "    op2b_cp_async_commit();",
+          "    if (t + 2 * step < p.rg_blocks) tn = p.rg_dir[t + 2 * step];",
+          "    op2b_cp_async_wait_but<1>();",
+          "    __syncthreads();",
+          "    {"]
+    L += _sums_parse(spec, "      ")
+    L.append("      for (int i = threadIdx.x; i < NE; i += %d) {" % bs)
+    if R["ids"]:
+        L.append("        const op2b_i64 e = elems[i];")
+    L += _sums_element(spec, "        ")
+    L += ["      }", "    }", "    __syncthreads();", "    {"]
+    L += _sums_parse(spec, "      ")
+    L += _sums_flush(spec, "      ")
+    L += ["    }", "  }"]
+    _gbl_epilogue(spec, L)
+    L.append("}")
+    return "\n".join(L)
+
+
 def _staged_flush(R, bs, ind):
     L = []
     for q, (slot, st, ctype, cdim) in enumerate(R["inc_pairs"]):
@@ -1053,6 +1265,8 @@ def _staged_body(spec):
     conflicts to the user)."""
     bs = spec.block_size
     R = spec.region
+    if R.get("sums"):
+        return _sums_body(spec)
     ns = len(R["stage_arity"])
     used = staged_used(spec)
     L = ["extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec))]

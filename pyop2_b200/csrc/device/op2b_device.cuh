@@ -60,6 +60,14 @@ __device__ __forceinline__ void op2b_cp_async_row(void *dst, const void *src) {
 
 __device__ __forceinline__ void op2b_cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// Copies issued since the last commit form a group; wait for all but the N
+// newest groups.
+__device__ __forceinline__ void op2b_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void op2b_cp_async_wait_but() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // Copy of n 16-byte units to shared memory by a CTA of THREADS threads.
 template <int THREADS>
 __device__ __forceinline__ void op2b_rb_copy(uint4 *dst, const uint4 *src, int n) {
@@ -192,6 +200,17 @@ __device__ __forceinline__ void op2b_cp_async_srow(void *base, int r, const void
   }
 }
 
+// cp.async of 16-byte chunk j of one row (of B bytes at src) into row r of a
+// staged array: with neighbouring lanes on the chunks of one row a warp's copy
+// names each row once.
+template <int B>
+__device__ __forceinline__ void op2b_cp_async_schunk(void *base, int r, int j, const void *src) {
+  static_assert(B % 16 == 0, "rows of whole chunks");
+  op2b_cp_async_row<16>(reinterpret_cast<char *>(base) + (op2b_i64)r * B +
+                            16 * op2b_srow_layout<B>::chunk(r, j),
+                        reinterpret_cast<const char *>(src) + 16 * j);
+}
+
 // SoA row: component k of element e lives at base[k * stride + e].
 template <typename T, int N>
 __device__ __forceinline__ void op2b_load_soa(T (&dst)[N], const T *__restrict__ base, op2b_i64 e,
@@ -250,6 +269,28 @@ template <typename T, int N>
 __device__ __forceinline__ void op2b_atomic_row(T *dst, const T (&v)[N]) {
 #pragma unroll
   for (int k = 0; k < N; ++k) op2b_atomic_add(dst + k, v[k]);
+}
+
+// Rows of a warp for adding to a Dat: lane l holds piece l mod K (VE values) of
+// row l / K, whose target is g.  In add i (of VE) the lane takes value c of a row:
+// whole rows from neighbouring lanes, so that a row of 32 bytes is one sector of
+// one request and not of two or four.
+template <int K, int VE, typename T>
+__device__ __forceinline__ T op2b_row_share(int i, const T (&s)[VE], int g, int &row, int &c, op2b_i64 &target) {
+  constexpr int C = K * VE;
+  static_assert(32 % C == 0, "rows of 1 to 32 values, a power of two");
+  const int lane = threadIdx.x & 31;
+  c = lane % C;
+  row = i * (32 / C) + lane / C;
+  const int from = row * K + c / VE;
+  T x = __shfl_sync(0xffffffffu, s[0], from);
+#pragma unroll
+  for (int v = 1; v < VE; ++v) {
+    const T y = __shfl_sync(0xffffffffu, s[v], from);
+    if (c % VE == v) x = y;
+  }
+  target = __shfl_sync(0xffffffffu, g, from);
+  return x;
 }
 
 // Record the first Mat insertion outside the Sparsity (PETSc raises

@@ -54,6 +54,10 @@ struct RegionPlan {
   int32_t *thrcol = nullptr, *nthrcol = nullptr;
   int16_t *loc = nullptr;
   int32_t max_nthrcol = 0;
+  // op2b_region_plan_packets
+  int2 *dir = nullptr;
+  uint4 *packets = nullptr;
+  int32_t max_elems = 0, max_packet = 0;
   std::vector<int32_t> max_count;   // per staged Map: largest tcnt over blocks
   std::vector<int32_t> arity;       // per staged Map: rows per element (loc rows from row_base)
   bool bank_slots = false;          // op2b_region_plan_bank_slots applied
@@ -491,6 +495,126 @@ __global__ void rg_slot_apply_kernel(int nstage, int set_size, const int32_t *__
   }
 }
 
+// Within each block of an evenly cut partition, the elements of one row-0 target
+// of the growth Map next to each other, in order of first use: lanes that read one
+// staged row share the access, and a target's contributions lie together.
+__global__ void __launch_bounds__(kRgStageThreads)
+rg_group_kernel(const int32_t *__restrict__ boff, const int32_t *__restrict__ map, int arity,
+                const int32_t *__restrict__ order, int32_t *__restrict__ out) {
+  extern __shared__ int32_t rg_group_smem[];      // [part_size] target, then first position
+  const int start = boff[blockIdx.x], ne = boff[blockIdx.x + 1] - start;
+  int32_t *tgt = rg_group_smem, *first = tgt + ne;
+  for (int i = threadIdx.x; i < ne; i += kRgStageThreads) tgt[i] = map[(int64_t)order[start + i] * arity];
+  __syncthreads();
+  for (int i = threadIdx.x; i < ne; i += kRgStageThreads) {
+    int j = 0;
+    while (tgt[j] != tgt[i]) ++j;
+    first[i] = j;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < ne; i += kRgStageThreads) {
+    int rank = 0;
+    for (int j = 0; j < ne; ++j) rank += first[j] < first[i] || (first[j] == first[i] && j < i);
+    out[start + rank] = order[start + i];
+  }
+}
+
+// Packets of the summing staged form: all a CTA needs to run a block, copied to
+// shared memory while the block before it runs.  In 16-byte units:
+//   {NE elements, 0, 0, 0}, {distinct targets of staged Maps 0..3}
+//   with ids: elements int32 [NE]
+//   per staged Map: targets int32 [nt]; rows uint16 [arity][NE], indices of
+//     targets; with inc: per target the end of its run in the list uint16 [nt],
+//     the list uint16 [arity * NE]: contribution row * NE + element, ascending
+// each part to a whole unit.
+struct RgPacket {
+  int32_t nstage, ids;
+  int32_t arity[4], row0[4], inc[4];
+};
+
+// 16-byte units of a packet.
+__host__ __device__ inline int rg_packet_units(const RgPacket &K, int ne, const int32_t *nt) {
+  int u = 2 + (K.ids ? (ne + 3) / 4 : 0);
+  for (int q = 0; q < K.nstage; ++q) {
+    u += (nt[q] + 3) / 4 + (ne * K.arity[q] + 7) / 8;
+    if (K.inc[q]) u += (nt[q] + 7) / 8 + (ne * K.arity[q] + 7) / 8;
+  }
+  return u;
+}
+
+// One CTA per block: the lists' counts and places by shared-memory atomics, each
+// target's few contributions sorted by its thread.
+__global__ void __launch_bounds__(kRgStageThreads)
+rg_packet_kernel(const RgPacket K, int set_size, const int32_t *__restrict__ boff,
+                 const int32_t *__restrict__ order, const int32_t *__restrict__ tcnt,
+                 const int32_t *__restrict__ toff, const int32_t *__restrict__ tlist,
+                 const int16_t *__restrict__ loc, const int2 *__restrict__ dir, uint4 *__restrict__ packets,
+                 int most) {
+  extern __shared__ int32_t rg_packet_smem[];     // [most] places, then [most] list
+  int32_t *place = rg_packet_smem, *list = place + most;
+  const int blk = blockIdx.x, tid = threadIdx.x;
+  const int start = boff[blk], ne = boff[blk + 1] - start;
+  const int32_t *nt = tcnt + blk * K.nstage;
+  uint4 *at = packets + dir[blk].x;
+  if (tid < 2) {
+    uint32_t h[4] = {tid ? 0u : (uint32_t)ne, 0u, 0u, 0u};
+    for (int q = 0; tid && q < K.nstage; ++q) h[q] = (uint32_t)nt[q];
+    at[tid] = make_uint4(h[0], h[1], h[2], h[3]);
+  }
+  at += 2;
+  if (K.ids) {
+    int32_t *elems = reinterpret_cast<int32_t *>(at);
+    for (int i = tid; i < ne; i += kRgStageThreads) elems[i] = order[start + i];
+    at += (ne + 3) / 4;
+  }
+  for (int q = 0; q < K.nstage; ++q) {
+    const int n = nt[q], nc = ne * K.arity[q];
+    const int32_t *from = tlist + toff[blk * K.nstage + q];
+    int32_t *targets = reinterpret_cast<int32_t *>(at);
+    for (int t = tid; t < n; t += kRgStageThreads) targets[t] = from[t];
+    at += (n + 3) / 4;
+    uint16_t *rows = reinterpret_cast<uint16_t *>(at);
+    const int16_t *l0 = loc + (int64_t)K.row0[q] * set_size + start;
+    auto target = [&](int c) { return (int)l0[(int64_t)(c / ne) * set_size + c % ne]; };
+    for (int c = tid; c < nc; c += kRgStageThreads) rows[c] = (uint16_t)target(c);
+    at += (nc + 7) / 8;
+    if (!K.inc[q]) continue;
+    __syncthreads();                              // the list before this one is read
+    for (int t = tid; t < n; t += kRgStageThreads) place[t] = 0;
+    __syncthreads();
+    for (int c = tid; c < nc; c += kRgStageThreads) atomicAdd(&place[target(c)], 1);
+    __syncthreads();
+    uint16_t *end = reinterpret_cast<uint16_t *>(at);
+    at += (n + 7) / 8;
+    uint16_t *out = reinterpret_cast<uint16_t *>(at);
+    at += (nc + 7) / 8;
+    int carry = 0;
+    for (int t0 = 0; t0 < n; t0 += kRgStageThreads) {
+      const int t = t0 + tid, mine = t < n ? place[t] : 0;
+      int tot;
+      const int pos = carry + block_excl_scan(mine, &tot);
+      if (t < n) {
+        place[t] = pos;
+        end[t] = (uint16_t)(pos + mine);
+      }
+      carry += tot;
+    }
+    __syncthreads();
+    for (int c = tid; c < nc; c += kRgStageThreads) list[atomicAdd(&place[target(c)], 1)] = c;
+    __syncthreads();
+    for (int t = tid; t < n; t += kRgStageThreads) {
+      const int last = place[t], first = t ? place[t - 1] : 0;
+      for (int i = first + 1; i < last; ++i) {
+        const int c = list[i];
+        int j = i;
+        for (; j > first && list[j - 1] > c; --j) list[j] = list[j - 1];
+        list[j] = c;
+      }
+      for (int i = first; i < last; ++i) out[i] = (uint16_t)list[i];
+    }
+  }
+}
+
 static int rg_grid(int64_t n) {
   return std::max(1, std::min(op2b_div_up(std::max<int64_t>(n, 1), kRgThreads), sm_count() * 8));
 }
@@ -504,15 +628,17 @@ static void region_release(RegionPlan *p, cudaStream_t s) {
   int32_t *arrs[] = {p->order, p->boff, p->tlist, p->toff, p->tcnt, p->thrcol, p->nthrcol};
   for (int32_t *a : arrs) dev_free(a, s);
   dev_free(p->loc, s);
+  dev_free(p->dir, s);
+  dev_free(p->packets, s);
   delete p;
 }
 
 extern "C" {
 
-int op2b_region_plan_build(int32_t set_size, int32_t part_size, int32_t region_size,
-                           uint64_t grow_map, int32_t grow_arity, int32_t grow_ntargets,
-                           int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
-                           const int32_t *stage_inc, uint64_t stream, uint64_t *plan_out) {
+static int region_plan_build(int32_t set_size, int32_t part_size, int32_t region_size,
+                             uint64_t grow_map, int32_t grow_arity, int32_t grow_ntargets,
+                             int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
+                             const int32_t *stage_inc, bool even, uint64_t stream, uint64_t *plan_out) {
   OP2B_REQUIRE_INIT();
   if (set_size < 0 || part_size <= 0 || region_size <= 0 || grow_arity <= 0 || grow_ntargets < 0 ||
       nstage < 0 || nstage > 64 || !plan_out ||
@@ -635,7 +761,9 @@ int op2b_region_plan_build(int32_t set_size, int32_t part_size, int32_t region_s
   // ---- blocks: every region cut into nearly equal runs of <= part_size
   std::vector<int32_t> h_boff;
   h_boff.push_back(0);
-  for (int r = 0; r < nregions; ++r) {
+  // (even: the whole order into runs of part_size)
+  for (int a = 0; even && a < n;) h_boff.push_back(a = std::min(n, a + part_size));
+  for (int r = 0; !even && r < nregions; ++r) {
     const int a = h_rstart[r], cnt = h_rstart[r + 1] - a;
     if (cnt <= 0) continue;
     const int pieces = op2b_div_up(cnt, part_size);
@@ -646,6 +774,17 @@ int op2b_region_plan_build(int32_t set_size, int32_t part_size, int32_t region_s
   RG_TRY(alloc((void **)&P->boff, sizeof(int32_t) * (nblocks + 1), false));
   RG_CUDA(cudaMemcpyAsync(P->boff, h_boff.data(), sizeof(int32_t) * (nblocks + 1),
                           cudaMemcpyHostToDevice, s));
+
+  if (even && nblocks > 0) {
+    const int gsmem = 2 * part_size * (int)sizeof(int32_t);
+    int32_t *grouped = nullptr;
+    RG_TRY(alloc((void **)&grouped, sizeof(int32_t) * n, true));
+    RG_CUDA(cudaFuncSetAttribute(rg_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gsmem));
+    rg_group_kernel<<<nblocks, kRgStageThreads, gsmem, s>>>(P->boff, gmap, grow_arity, P->order, grouped);
+    RG_CUDA(cudaGetLastError());
+    temps.back() = P->order;
+    P->order = grouped;
+  }
 
   // ---- staging lists of every staged Map
   RG_TRY(alloc((void **)&P->tcnt, sizeof(int32_t) * (size_t)nblocks * nstage, false));
@@ -752,6 +891,22 @@ int op2b_region_plan_build(int32_t set_size, int32_t part_size, int32_t region_s
   return OP2B_OK;
 }
 
+int op2b_region_plan_build(int32_t set_size, int32_t part_size, int32_t region_size,
+                           uint64_t grow_map, int32_t grow_arity, int32_t grow_ntargets,
+                           int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
+                           const int32_t *stage_inc, uint64_t stream, uint64_t *plan_out) {
+  return region_plan_build(set_size, part_size, region_size, grow_map, grow_arity, grow_ntargets, nstage,
+                           stage_map, stage_arity, stage_inc, false, stream, plan_out);
+}
+
+int op2b_region_plan_build_even(int32_t set_size, int32_t part_size, int32_t region_size,
+                                uint64_t grow_map, int32_t grow_arity, int32_t grow_ntargets,
+                                int32_t nstage, const uint64_t *stage_map, const int32_t *stage_arity,
+                                const int32_t *stage_inc, uint64_t stream, uint64_t *plan_out) {
+  return region_plan_build(set_size, part_size, region_size, grow_map, grow_arity, grow_ntargets, nstage,
+                           stage_map, stage_arity, stage_inc, true, stream, plan_out);
+}
+
 int op2b_region_plan_info(uint64_t plan, int32_t *nblocks, int32_t *nregions, int32_t *levels,
                           int32_t *max_count, int64_t *tlist_len, int32_t *max_nthrcol) {
   RegionPlan *P = reinterpret_cast<RegionPlan *>(plan);
@@ -776,6 +931,82 @@ int op2b_region_plan_array(uint64_t plan, int32_t which, uint64_t *dptr, int64_t
   if (which < 0 || which > 7) return set_error(OP2B_ERR_ARG, "region plan array %d", which);
   *dptr = reinterpret_cast<uint64_t>(ptrs[which]);
   if (count) *count = counts[which];
+  return OP2B_OK;
+}
+
+int op2b_region_plan_packets(uint64_t plan, const int32_t *stage_inc, int32_t ids, uint64_t stream,
+                             uint64_t *dir, uint64_t *packets, int32_t *max_elems, int32_t *max_packet) {
+  OP2B_REQUIRE_INIT();
+  RegionPlan *P = reinterpret_cast<RegionPlan *>(plan);
+  if (!P || !dir || !packets || !max_elems || !max_packet || (P->nstage > 0 && !stage_inc) || P->nstage > 4)
+    return set_error(OP2B_ERR_ARG, "op2b_region_plan_packets: null argument or more than 4 staged Maps");
+  if (P->bank_slots) return set_error(OP2B_ERR_STATE, "op2b_region_plan_packets: padded slots");
+  cudaStream_t s = stream_of(stream);
+  if (!P->packets) {
+    const int nb = P->nblocks, ns = P->nstage;
+    const size_t nbs = (size_t)nb * ns;
+    RgPacket K = {};
+    K.nstage = ns;
+    K.ids = ids != 0;
+    for (int q = 0, r = 0; q < ns; r += P->arity[q++]) {
+      K.arity[q] = P->arity[q];
+      K.row0[q] = r;
+      K.inc[q] = stage_inc[q] != 0;
+    }
+    std::vector<int32_t> h_boff(nb + 1, 0), h_cnt(std::max<size_t>(nbs, 1));
+    if (nb) OP2B_CUDA(cudaMemcpyAsync(h_boff.data(), P->boff, sizeof(int32_t) * (nb + 1), cudaMemcpyDeviceToHost, s));
+    if (nbs) OP2B_CUDA(cudaMemcpyAsync(h_cnt.data(), P->tcnt, sizeof(int32_t) * nbs, cudaMemcpyDeviceToHost, s));
+    OP2B_CUDA(cudaStreamSynchronize(s));
+    std::vector<int2> h_dir(nb + 1);
+    int64_t units = 0;
+    int most = 1, room = 2, elems = 0;
+    for (int b = 0; b < nb; ++b) {
+      const int ne = h_boff[b + 1] - h_boff[b];
+      elems = std::max(elems, ne);
+      for (int q = 0; q < ns; ++q)
+        if (K.inc[q]) most = std::max(most, std::max(ne * K.arity[q], h_cnt[(size_t)b * ns + q]));
+      const int u = rg_packet_units(K, ne, &h_cnt[(size_t)b * ns]);
+      h_dir[b] = make_int2((int)units, u);
+      room = std::max(room, u);
+      units += u;
+    }
+    const int smem = 2 * most * (int)sizeof(int32_t);
+    if (most > 65535 || smem > smem_optin() || units > INT_MAX)
+      return set_error(OP2B_ERR_ARG, "op2b_region_plan_packets: %d contributions in a block, %lld units", most,
+                       (long long)units);
+    int2 *d_dir = nullptr;
+    uint4 *d_pk = nullptr;
+    int rc = dev_alloc((void **)&d_dir, sizeof(int2) * (nb + 1), s);
+    if (!rc) rc = dev_alloc((void **)&d_pk, sizeof(uint4) * (size_t)std::max<int64_t>(units, 1), s);
+    if (!rc)
+      rc = check_cuda(cudaMemcpyAsync(d_dir, h_dir.data(), sizeof(int2) * (nb + 1), cudaMemcpyHostToDevice, s),
+                      "op2b_region_plan_packets copy");
+    if (!rc) rc = check_cuda(cudaMemsetAsync(d_pk, 0, sizeof(uint4) * (size_t)std::max<int64_t>(units, 1), s),
+                             "op2b_region_plan_packets memset");
+    if (!rc)
+      rc = check_cuda(cudaFuncSetAttribute(rg_packet_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                      "rg_packet_kernel shared memory");
+    if (!rc && nb > 0) {
+      rg_packet_kernel<<<nb, kRgStageThreads, smem, s>>>(K, P->set_size, P->boff, P->order, P->tcnt, P->toff,
+                                                         P->tlist, P->loc, d_dir, d_pk, most);
+      rc = check_cuda(cudaGetLastError(), "rg_packet_kernel");
+    }
+    // the host directory ends here
+    const int rs = check_cuda(cudaStreamSynchronize(s), "op2b_region_plan_packets");
+    if (rc || rs) {
+      dev_free(d_dir, s);
+      dev_free(d_pk, s);
+      return rc ? rc : rs;
+    }
+    P->dir = d_dir;
+    P->packets = d_pk;
+    P->max_elems = elems;
+    P->max_packet = room;
+  }
+  *dir = reinterpret_cast<uint64_t>(P->dir);
+  *packets = reinterpret_cast<uint64_t>(P->packets);
+  *max_elems = P->max_elems;
+  *max_packet = P->max_packet;
   return OP2B_OK;
 }
 
