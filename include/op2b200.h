@@ -449,17 +449,17 @@ int op2b_mat_zero_rows(uint64_t vals, uint64_t rowptr, uint64_t colidx, int32_t 
  * values must lie in their target Sets.  Replaces the colouring and the
  * LMA-to-CSR scatter of such a loop (pyop2/plan.pyx:214-376,
  * assets/cuda_matrix_support.jinja2:27-81).
- * Block b's packet starts at 16 * dir[b].start bytes of packets and takes
- * 16 * dir[b].size (dir: int32 pairs).  It holds int32 {elements NE, short
- * entries, long entries, items NI}, int32 {targets of each staged Map}, then,
- * each padded to 16 bytes: elements int32 [NE] (if ids); items uint16 [ra][NE]
- * ((element, map index) landing in the block's rows, else NI); per staged Map
- * targets int32 and indices into them uint16 [arity][NE]; short entries uint32
- * {CSR position, contribution | second contribution << 16
- * (ca * NS: none)}; long entries uint32 {position, first | last + 1 << 16
- * in the list}; the list uint16.  A contribution is c * NS + item, NS
- * the first odd number above NI.
- * max_targets: 4 values; max_packet in 16-byte units.
+ * Block b's packet starts at unit dir[b].x of packets (units of 16 bytes); the low
+ * 16 bits of dir[b].y are the unit its short entries start at, the high 16 its
+ * size.  It holds int32 {elements NE, short entries, long entries, items NI}, int32
+ * {targets of each staged Map}, then, each padded to a unit: elements int32 [NE]
+ * (if ids); items uint16 [ra][NE] ((element, map index) landing in the block's
+ * rows, else NI); per staged Map targets int32 and indices into them uint16
+ * [arity][NE]; long entries uint32 {CSR position, first | last + 1 << 16 in the
+ * list}; the list uint16; short entries uint32 {position, contribution | second
+ * contribution << 16 (ca * NS: none)}.  A contribution is c * NS + item, NS the
+ * first odd number above NI.
+ * max_targets: 4 values; max_packet: most units before the short entries.
  * ---------------------------------------------------------------------- */
 int op2b_row_blocks_build(uint64_t rmap, uint64_t cmap, int32_t nelem, int32_t ra, int32_t ca,
                           int32_t nrows, uint64_t rowptr, uint64_t colidx, int32_t region,

@@ -1486,8 +1486,7 @@ def _rowblk_parse(spec, ind):
         L.append("%sconst unsigned short *lx%d = (const unsigned short *)(tl%d + ((nt%d + 3) & ~3));"
                  % (ind, st, st, st))
         at = "(const int *)(lx%d + ((NE * %d + 7) & ~7))" % (st, R["stage_arity"][st])
-    L += ["%sconst uint2 *shorts = (const uint2 *)(%s);" % (ind, at),
-          "%sconst uint2 *longs = shorts + ((nshort + 1) & ~1);" % ind,
+    L += ["%sconst uint2 *longs = (const uint2 *)(%s);" % (ind, at),
           "%sconst unsigned short *ids = (const unsigned short *)(longs + ((nlong + 1) & ~1));" % ind]
     off = "op2b_smem + 16 * room"
     for q, (slot, st, ct, c) in enumerate(R["read_pairs"]):
@@ -1544,14 +1543,17 @@ def _rowblk_body(spec):
     The element form adds every local entry with a reduction of its own into
     L2 (139 G/s, its bound); here rows are runs of sectors written once.
     Measured on a B200, the loop with the memsets of its Mats: P2 K + M
-    1024 x 1024 in FP64 605 us (element form 1028), P2 512 x 512 with FP32
-    element math and compensated sums 143 us (two phases through memory 344),
-    P1 mass of 1.0 M elements 39 us (60).  What bounds it: shared memory
-    wavefronts (about 60 % of their rate on P2: 4 loads and 2 stores an entry,
-    72 stores an element) and the latency of a block's dependent steps at the
-    16 to 28 warps its shared memory allows.  Blocks of 8 to 20 KB of
-    contributions measured within 10 %; a ring of packets copied two blocks
-    ahead did not pay for its shared memory.
+    1024 x 1024 in FP64 548 us (element form 1028), P2 512 x 512 with FP32
+    element math and compensated sums 141 us (two phases through memory 344),
+    P1 mass of 1.0 M elements 35 us (51).  The short entries, half of a packet,
+    are read from L2, four at a time ahead of their use: as part of the packet
+    in shared memory they took 607, 145 and 35 us.  What bounds it: shared
+    memory wavefronts (about 60 % of their rate on P2: 4 loads and 2 stores an
+    entry, 36 stores of both Mats an element) and the latency of a block's
+    dependent steps at the 16 to 32 warps its shared memory and registers allow.
+    Blocks of 8 to 20 KB of contributions measured 708, 609, 565 and 546 us on
+    P2 1024 x 1024 and 66, 63, 63 and 64 on the P1 mesh with its right-hand side;
+    a ring of packets copied two blocks ahead did not pay for its shared memory.
 
     ``spec.rowblk``: ra, ca, kahan, and map_stage, stage_arity and read_pairs
     as in the staged form."""
@@ -1566,12 +1568,16 @@ def _rowblk_body(spec):
     L.append("  op2b_i64 t = blockIdx.x;")
     L.append("  int2 td = p.rb_dir[t], tn = td;")
     L.append("  if (t + step < p.rb_blocks) tn = p.rb_dir[t + step];")
+    L.append("  op2b_rb_prefetch<%d>(p.rb_pkt + td.x + (td.y & 0xffff), "
+             "(int)((unsigned)td.y >> 16) - (td.y & 0xffff));" % bs)
     L.append("  for (; t < p.rb_blocks; t += step) {")
-    L.append("    op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rb_pkt + td.x, td.y);" % bs)
+    L.append("    op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rb_pkt + td.x, td.y & 0xffff);" % bs)
+    L.append("    const uint2 *shorts = (const uint2 *)(p.rb_pkt + td.x + (td.y & 0xffff));")
     # the directory is read two blocks ahead, so no thread waits for it
     L.append("    td = tn;")
     L.append("    if (t + 2 * step < p.rb_blocks) tn = p.rb_dir[t + 2 * step];")
-    L.append("    if (t + step < p.rb_blocks) op2b_rb_prefetch<%d>(p.rb_pkt + td.x, td.y);" % bs)
+    L.append("    if (t + step < p.rb_blocks) op2b_rb_prefetch<%d>(p.rb_pkt + td.x, "
+             "(unsigned)td.y >> 16);" % bs)
     L.append("    op2b_cp_async_wait();")
     L.append("    __syncthreads();")
     L += _rowblk_parse(spec, "    ")
@@ -1597,7 +1603,6 @@ def _rowblk_body(spec):
         L.append("      const op2b_i64 e = elems[i];")
     L += _rowblk_element(spec, "      ")
     L.append("    }")
-    L.append("    __syncthreads();")
     L += _rowblk_sums(spec)
     L.append("    __syncthreads();     // the next packet takes this one's place")
     L.append("  }")
@@ -1607,7 +1612,7 @@ def _rowblk_body(spec):
 
 def _rowblk_sums(spec):
     """The block's entries: those of one or two contributions without a loop
-    over contributions (most entries of an element method's matrix), two at
+    over contributions (most entries of an element method's matrix), four at
     a time per thread; then the longer ones, which would hold up their warps."""
     bs, R = spec.block_size, spec.rowblk
     kahan = R["kahan"]
@@ -1619,8 +1624,7 @@ def _rowblk_sums(spec):
         return "%s += %s;" % (v, s)
 
     def load(u, ind):
-        return ["%sconst uint2 w%s = shorts[l%s];" % (ind, u, u)] + [
-            "%s%s v%d%s = p.mz%d ? (%s)0 : p.mv%d[w%s.x];" % (ind, t, j, u, j, t, j, u) for j, t in mats]
+        return ["%s%s v%d%s = p.mz%d ? (%s)0 : p.mv%d[w%s.x];" % (ind, t, j, u, j, t, j, u) for j, t in mats]
 
     def sums(u, ind):
         L = ["%sconst op2b_rb_sum s%s = S[w%s.y & 0xffffu];" % (ind, u, u)]
@@ -1637,15 +1641,30 @@ def _rowblk_sums(spec):
 
     def store(u, ind):
         return ["%sp.mv%d[w%s.x] = v%d%s;" % (ind, j, u, j, u) for j, t in mats]
+    # the short entries come from global memory (fetched into L2 a block ahead),
+    # the next four of a thread while it adds four
+    names = "abcd"
+
+    def fetch(var, ind, ahead):
+        return ["%sif (l + %d < nshort) %s_%s = __ldg(shorts + l + %d);" % (
+            ind, (k + ahead) * bs, var, u, (k + ahead) * bs) for k, u in enumerate(names)]
     L = ["    {",
          "      int l = threadIdx.x;",
-         "      for (; l + %d < nshort; l += %d) {" % (bs, 2 * bs),
-         "        const int l_a = l, l_b = l + %d;" % bs]
-    for part in (load, sums, store):
-        L += part("_a", "        ") + part("_b", "        ")
-    L += ["      }", "      if (l < nshort) {"]
-    for part in (load, sums, store):
-        L += part("", "        ")
+         "      const uint2 none = make_uint2(0, (unsigned)(NS * %d) * 0x10001u);" % R["ca"],
+         "      uint2 %s;" % ", ".join("w_%s = none" % u for u in names)]
+    L += fetch("w", "      ", 0)
+    L += ["      __syncthreads();",
+          "      for (; l < nshort; l += %d) {" % (len(names) * bs),
+          "        uint2 %s;" % ", ".join("n_%s = none" % u for u in names)]
+    L += fetch("n", "        ", len(names))
+    for part in (load, sums):
+        for u in names:
+            L += part("_" + u, "        ")
+    for k, u in enumerate(names):
+        L.append("        if (l + %d < nshort) {" % (k * bs))
+        L += store("_" + u, "          ")
+        L.append("        }")
+    L.append("        " + " ".join("w_%s = n_%s;" % (u, u) for u in names))
     L += ["      }",
           "      for (int l = threadIdx.x; l < nlong; l += %d) {" % bs,
           "        const uint2 w = longs[l];"]

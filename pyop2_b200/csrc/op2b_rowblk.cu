@@ -31,13 +31,13 @@
 //      per staged Map (the loop reads Dats through it): targets int32 [nt],
 //              the block's distinct targets in order of first use, and
 //              lidx uint16 [arity][NE], each element's targets in that list
-//      shorts  per entry of one or two contributions, rows in order, columns
-//              in order: {CSR position, first contribution | second << 16}; an
-//              entry of one has ca * NS as its second, a place the stub fills
-//              with -0.0
-//      longs   per other entry: {CSR position, first | last + 1 << 16 of its
-//              contributions in list} (apart: a warp waits for its longest)
+//      longs   per entry of three or more contributions: {CSR position,
+//              first | last + 1 << 16 of its contributions in list}
 //      list    uint16: the long entries' contributions
+//    and, which the CTA reads from where it lies,
+//      shorts  per other entry, rows in order, columns in order: {CSR position,
+//              first contribution | second << 16}; an entry of one has ca * NS
+//              as its second, a place the stub fills with -0.0
 //    A contribution is its place in the block's shared array [ca][NS], NS the
 //    first odd number above NI: c * NS + item (column NI takes what other
 //    blocks own); each part is padded to 16 bytes, and an entry's contributions
@@ -61,9 +61,10 @@ constexpr int kRbMaxKeys = 8192;       // items of a block, and map entries of i
 constexpr int kRbMaxContrib = 16384;   // contributions of a block
 
 struct RowBlocks {
-  int32_t nblocks = 0, max_items = 0, max_packet = 0;    // max_packet: 16-byte units
+  int32_t nblocks = 0, max_items = 0;
+  int32_t max_packet = 0;      // 16-byte units, without the short entries
   int32_t max_targets[kRbStages] = {0, 0, 0, 0};
-  int2 *dir = nullptr;         // [nblocks] packet start and size, 16-byte units
+  int2 *dir = nullptr;         // [nblocks] packet start, first | size << 16, 16-byte units
   uint4 *pkt = nullptr;
 };
 
@@ -431,14 +432,15 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
   const int nshort = ne - nlong - nempty;
   __shared__ int s_start;
   const int u_elems = A.ids ? rb_units(4 * NE) : 0, u_items = rb_units(2 * ra * NE), u_shorts = rb_units(8LL * nshort), u_longs = rb_units(8LL * nlong);
-  int total = 2 + u_elems + u_items + u_shorts + u_longs + rb_units(2LL * nlids);
-  for (int s = 0; s < A.st.n; ++s) total += rb_units(4 * nt[s]) + rb_units(2 * A.st.arity[s] * NE);
+  int head = 2 + u_elems + u_items + u_longs + rb_units(2LL * nlids);
+  for (int s = 0; s < A.st.n; ++s) head += rb_units(4 * nt[s]) + rb_units(2 * A.st.arity[s] * NE);
+  const int total = head + u_shorts;
   if (tid == 0) {
     s_start = atomicAdd(&A.scal[kSCursor], total);
-    A.dir[blk] = make_int2(s_start, total);
-    atomicMax(&A.scal[kSMaxPacket], total);
+    A.dir[blk] = make_int2(s_start, (int)((unsigned)head | (unsigned)total << 16));
+    atomicMax(&A.scal[kSMaxPacket], head);
     for (int s = 0; s < A.st.n; ++s) atomicMax(&A.scal[kSMaxTargets + s], nt[s]);
-    if ((int64_t)ns * ca > 65535) atomicExch(&A.scal[kSFlag], 1);
+    if ((int64_t)ns * ca > 65535 || total > 65535) atomicExch(&A.scal[kSFlag], 1);
   }
   __syncthreads();
   if ((int64_t)s_start + total > A.cap) return;    // the host allocates what the cursor says and repeats
@@ -462,8 +464,8 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
     P += rb_units(2 * a * NE);
     at += a;
   }
-  uint2 *shorts = reinterpret_cast<uint2 *>(P), *longs = reinterpret_cast<uint2 *>(P + u_shorts);
-  unsigned short *ids = reinterpret_cast<unsigned short *>(P + u_shorts + u_longs);
+  uint2 *longs = reinterpret_cast<uint2 *>(P), *shorts = reinterpret_cast<uint2 *>(A.pkt + s_start + head);
+  unsigned short *ids = reinterpret_cast<unsigned short *>(P + u_longs);
   int sc = 0, lc = 0, ic = 0, found = 0;
   for (int base = 0; base < ne; base += kRbThreads) {
     const int j = base + tid;
