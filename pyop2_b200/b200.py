@@ -1214,7 +1214,7 @@ class RowBlocks(object):
 # threads per CTA of the row block stubs, and bytes of contributions to one Mat
 # a block aims at (its region's elements times the bytes of one element)
 _ROWBLK_THREADS = 128
-_ROWBLK_BYTES = 20 << 10
+_ROWBLK_BYTES = 18 << 10
 
 
 # contributions a launch adds, below which the form makes no difference worth

@@ -1461,7 +1461,7 @@ def rowblk_smem(spec, max_items, max_packet, max_targets):
     rows, and the contributions of a block, [ca][odd number of items], with
     one place of zeros."""
     R = spec.rowblk
-    nb = 16 * max_packet
+    nb = 32 * max_packet
     for slot, st, ctype, cdim in R["read_pairs"]:
         nb += (max_targets[st] * cdim * _CSIZE[ctype] + 15) // 16 * 16
     return nb + (((max_items + 1) | 1) * R["ca"] + 1) * _rowblk_sum_decl(spec)[1]
@@ -1488,7 +1488,7 @@ def _rowblk_parse(spec, ind):
         at = "(const int *)(lx%d + ((NE * %d + 7) & ~7))" % (st, R["stage_arity"][st])
     L += ["%sconst uint2 *longs = (const uint2 *)(%s);" % (ind, at),
           "%sconst unsigned short *ids = (const unsigned short *)(longs + ((nlong + 1) & ~1));" % ind]
-    off = "op2b_smem + 16 * room"
+    off = "op2b_smem + 32 * room"
     for q, (slot, st, ct, c) in enumerate(R["read_pairs"]):
         L.append("%s%s *rd%d = (%s *)(%s);" % (ind, ct, q, ct, off))
         off = "(unsigned char *)rd%d + ((nt%d * %d + 15) & ~15)" % (q, st, c * _CSIZE[ct])
@@ -1529,9 +1529,9 @@ def _rowblk_element(spec, ind):
 
 def _rowblk_body(spec):
     """Increments by the owners of the rows: a persistent grid walks the row
-    blocks (op2b_row_blocks_build).  Per block the CTA copies the block's
-    packet (cp.async, 16 bytes a time; the next one is fetched into L2
-    meanwhile), then the distinct rows read through staged Maps, to shared
+    blocks (op2b_row_blocks_build).  Per block the CTA has the block's packet in
+    shared memory (copied with cp.async, 16 bytes a time, while the block before
+    runs), copies the distinct rows read through staged Maps to shared
     memory; a thread evaluates whole elements, each local entry that lands in
     the block's rows into the contributions S ([ca][items]: consecutive threads
     on consecutive places; what lands in another block's rows goes to a column
@@ -1543,17 +1543,18 @@ def _rowblk_body(spec):
     The element form adds every local entry with a reduction of its own into
     L2 (139 G/s, its bound); here rows are runs of sectors written once.
     Measured on a B200, the loop with the memsets of its Mats: P2 K + M
-    1024 x 1024 in FP64 548 us (element form 1028), P2 512 x 512 with FP32
-    element math and compensated sums 141 us (two phases through memory 344),
+    1024 x 1024 in FP64 520 us (element form 1028), P2 512 x 512 with FP32
+    element math and compensated sums 138 us (two phases through memory 344),
     P1 mass of 1.0 M elements 35 us (51).  The short entries, half of a packet,
-    are read from L2, four at a time ahead of their use: as part of the packet
-    in shared memory they took 607, 145 and 35 us.  What bounds it: shared
-    memory wavefronts (about 60 % of their rate on P2: 4 loads and 2 stores an
-    entry, 36 stores of both Mats an element) and the latency of a block's
-    dependent steps at the 16 to 32 warps its shared memory and registers allow.
-    Blocks of 8 to 20 KB of contributions measured 708, 609, 565 and 546 us on
-    P2 1024 x 1024 and 66, 63, 63 and 64 on the P1 mesh with its right-hand side;
-    a ring of packets copied two blocks ahead did not pay for its shared memory.
+    are read from L2, four at a time ahead of their use (as part of the packet
+    in shared memory: 607, 145 and 35 us); the packet copied a block ahead and
+    not when its block starts took P2 1024 from 548 to 520 us.  What bounds it:
+    shared memory wavefronts (about 60 % of their rate on P2: 4 loads and 2
+    stores an entry, 36 stores of both Mats an element) and the latency of a
+    block's dependent steps at the 16 to 28 warps its shared memory and
+    registers allow.  Blocks of 8, 12, 16, 18 and 20 KB of contributions measured
+    649, 565, 529, 518 and 539 us on P2 1024 x 1024, 146, 134, 141, 137 and 146
+    on P2 512 x 512 in FP32, and 62 to 64 on the P1 mesh with its right-hand side.
 
     ``spec.rowblk``: ra, ca, kahan, and map_stage, stage_arity and read_pairs
     as in the staged form."""
@@ -1562,24 +1563,21 @@ def _rowblk_body(spec):
     L.append("extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec)))
     _gbl_prologue(spec, L)
     L.append("  extern __shared__ __align__(16) unsigned char op2b_smem[];")
-    L.append("  const uint4 *pk = (const uint4 *)op2b_smem;")
-    L.append("  const int room = p.col_n;   // 16-byte units of a packet")
-    L.append("  const op2b_i64 step = gridDim.x;")
-    L.append("  op2b_i64 t = blockIdx.x;")
-    L.append("  int2 td = p.rb_dir[t], tn = td;")
-    L.append("  if (t + step < p.rb_blocks) tn = p.rb_dir[t + step];")
-    L.append("  op2b_rb_prefetch<%d>(p.rb_pkt + td.x + (td.y & 0xffff), "
-             "(int)((unsigned)td.y >> 16) - (td.y & 0xffff));" % bs)
-    L.append("  for (; t < p.rb_blocks; t += step) {")
-    L.append("    op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rb_pkt + td.x, td.y & 0xffff);" % bs)
-    L.append("    const uint2 *shorts = (const uint2 *)(p.rb_pkt + td.x + (td.y & 0xffff));")
-    # the directory is read two blocks ahead, so no thread waits for it
-    L.append("    td = tn;")
-    L.append("    if (t + 2 * step < p.rb_blocks) tn = p.rb_dir[t + 2 * step];")
-    L.append("    if (t + step < p.rb_blocks) op2b_rb_prefetch<%d>(p.rb_pkt + td.x, "
-             "(unsigned)td.y >> 16);" % bs)
-    L.append("    op2b_cp_async_wait();")
-    L.append("    __syncthreads();")
+    L += ["  const int room = p.col_n;   // 16-byte units of a packet",
+          "  const op2b_i64 step = gridDim.x;",
+          "  op2b_i64 t = blockIdx.x;",
+          # the directory is read two blocks ahead, so no thread waits for it
+          "  int2 td = p.rb_dir[t], tn = td;",
+          "  op2b_rb_copy<%d>((uint4 *)op2b_smem, p.rb_pkt + td.x, td.y & 0xffff);" % bs,
+          "  op2b_rb_prefetch<%d>(p.rb_pkt + td.x + (td.y & 0xffff), "
+          "(int)((unsigned)td.y >> 16) - (td.y & 0xffff));" % bs,
+          "  if (t + step < p.rb_blocks) tn = p.rb_dir[t + step];",
+          "  for (int odd = 0; t < p.rb_blocks; t += step, odd ^= 1) {",
+          "    const uint2 *shorts = (const uint2 *)(p.rb_pkt + td.x + (td.y & 0xffff));",
+          "    td = tn;",
+          "    op2b_cp_async_wait();",
+          "    __syncthreads();         // the packet is here, and the block before is done",
+          "    const uint4 *pk = (const uint4 *)op2b_smem + odd * room;"]
     L += _rowblk_parse(spec, "    ")
     if R["read_pairs"]:
         for st in range(len(R["stage_arity"])):
@@ -1596,15 +1594,22 @@ def _rowblk_body(spec):
                     L.append("      for (int k = 0; k < %d; ++k) rd%d[r * %d + k] = p.d%d[g * %d + k];"
                              % (c, q, c, slot, c))
             L.append("    }")
-        L.append("    op2b_cp_async_wait();")
-        L.append("    __syncthreads();")
+    L += ["    op2b_cp_async_commit();",
+          "    if (t + step < p.rb_blocks) {",
+          "      op2b_rb_copy<%d>((uint4 *)op2b_smem + (odd ^ 1) * room, p.rb_pkt + td.x, td.y & 0xffff);" % bs,
+          "      op2b_rb_prefetch<%d>(p.rb_pkt + td.x + (td.y & 0xffff), "
+          "(int)((unsigned)td.y >> 16) - (td.y & 0xffff));" % bs,
+          "    }",
+          "    op2b_cp_async_commit();",
+          "    if (t + 2 * step < p.rb_blocks) tn = p.rb_dir[t + 2 * step];"]
+    if R["read_pairs"]:
+        L += ["    op2b_cp_async_wait_but<1>();", "    __syncthreads();"]
     L.append("    for (int i = threadIdx.x; i < NE; i += %d) {" % bs)
     if any(a.kind == "direct" for a in spec.args):
         L.append("      const op2b_i64 e = elems[i];")
     L += _rowblk_element(spec, "      ")
     L.append("    }")
     L += _rowblk_sums(spec)
-    L.append("    __syncthreads();     // the next packet takes this one's place")
     L.append("  }")
     L.append("}")
     return "\n".join(L)
