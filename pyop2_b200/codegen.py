@@ -105,7 +105,8 @@ class LoopSpec(object):
         # staged form over a locality partition (mode 'staged'): map_stage
         # {map slot: staged Map}, stage_arity, row_base (first loc row of each
         # staged Map), read_pairs / inc_pairs [(Dat slot, staged Map, ctype,
-        # cdim)] staged / accumulated in shared memory
+        # cdim)] staged / accumulated in shared memory; sums: contributions
+        # stored and summed per target, ids: with the elements' ids in the packets
         self.region = None
         self.kernel_name = kernel_name
         self.kernel_code = kernel_code

@@ -22,11 +22,12 @@ keys of the B200 backend:
   between runs within rounding) or ``'lma'`` (two phases: the stub stores
   every contribution, then each target adds its contributions in element
   order -- the sequential backend's order -- optionally Kahan-compensated;
-  deterministic and independent of the launch configuration; loops it cannot
-  run fall back to ``'color'``) or ``'staged'`` (one launch over a locality
+  deterministic and independent of the launch configuration; large scalar Mat
+  assembly adds them in the same order by row blocks, without the store;
+  loops it cannot run fall back to ``'color'``) or ``'staged'`` (one launch over a locality
   partition: the set is reordered into compact regions grown on the GPU,
   each block's distinct targets are staged in shared memory and INC rows
-  accumulated there, then added once per target with atomics; summation
+  summed there, then added once per target with atomics; summation
   order varies between runs within rounding; loops without indirect INC,
   with Mats, or whose staged rows would not fit a CTA's shared memory run
   as ``'atomic'``) or ``'gather'`` (loops whose only writes are INC into
@@ -38,10 +39,12 @@ keys of the B200 backend:
   neighbouring targets; other loops run as with ``'staged'``);
 * ``region_size``: elements per region (one hashed seed per about this many
   elements) of the staged form's locality partition (0: half the partition
-  size, whose default in the staged form is 384);
-* ``staged_block_size``: threads per CTA of the staged form's stubs (one
-  CTA per block of the partition);
-* ``staged_tl_regs``: the staged stubs load their block's target ids into
+  size, whose default in the staged form is 384; where contributions are
+  summed per target instead of colour by colour, 5/4 of the 256 or 128
+  elements of a block);
+* ``staged_block_size``: threads per CTA of the staged form's stubs;
+* ``staged_tl_regs``: (this and the next two select the staged form that adds
+  colour by colour, which they tune) the staged stubs load their block's target ids into
   registers once (with the element rows) and reuse them for the row copies
   and the flush, which then adds one accumulated row per thread;
 * ``staged_bank_slots``: renumber the staged rows of each block of the
@@ -66,7 +69,11 @@ keys of the B200 backend:
   (the index becomes a run-time value per lane);
 * ``kahan``: compensated (Kahan) summation of owner-computes and two-phase
   (``inc_mode='lma'``) accumulation;
-* ``mat_slots``: assemble scalar Mats in the atomic form through a cached
+* ``mat_slots``: (with this, ``mat_per_entry``, ``mat_slots_rel`` and
+  ``itspace_split`` at their defaults, large scalar Mat assembly that keeps
+  running, or is about to be recorded in a graph, is run by the owners of the
+  rows instead: every stored entry written once, its contributions added in
+  element order) assemble scalar Mats in the atomic form through a cached
   scatter-slot table (the CSR position of every element's local entries,
   built once per Sparsity and Map pair: nelem x arity^2 int32 of device
   memory) instead of searching the CSR row for every entry;
