@@ -14,7 +14,8 @@
 //    scheduling;
 //  * order: elements sorted by (region, level, element id);
 //  * blocks: each region cut into nearly equal runs of at most part_size
-//    elements;
+//    elements, or (even) the whole order into runs of part_size, the elements
+//    of one target next to each other within a run;
 //  * staging: per block and staged Map the distinct targets over all Map
 //    rows in order of first use (tlist / toff / tcnt) and, per position of
 //    the reordered set and Map row, the target's index in that list (loc,
@@ -501,20 +502,35 @@ __global__ void rg_slot_apply_kernel(int nstage, int set_size, const int32_t *__
 __global__ void __launch_bounds__(kRgStageThreads)
 rg_group_kernel(const int32_t *__restrict__ boff, const int32_t *__restrict__ map, int arity,
                 const int32_t *__restrict__ order, int32_t *__restrict__ out) {
-  extern __shared__ int32_t rg_group_smem[];      // [part_size] target, then first position
+  extern __shared__ int32_t rg_group_smem[];      // [part_size] target, first position, count
   const int start = boff[blockIdx.x], ne = boff[blockIdx.x + 1] - start;
-  int32_t *tgt = rg_group_smem, *first = tgt + ne;
-  for (int i = threadIdx.x; i < ne; i += kRgStageThreads) tgt[i] = map[(int64_t)order[start + i] * arity];
+  int32_t *tgt = rg_group_smem, *first = tgt + ne, *count = first + ne;
+  for (int i = threadIdx.x; i < ne; i += kRgStageThreads) {
+    tgt[i] = map[(int64_t)order[start + i] * arity];
+    count[i] = 0;
+  }
   __syncthreads();
   for (int i = threadIdx.x; i < ne; i += kRgStageThreads) {
     int j = 0;
     while (tgt[j] != tgt[i]) ++j;
     first[i] = j;
+    atomicAdd(&count[j], 1);
+  }
+  __syncthreads();
+  // count: where each group starts
+  int carry = 0;
+  for (int i0 = 0; i0 < ne; i0 += kRgStageThreads) {
+    const int i = i0 + threadIdx.x;
+    int total;
+    const int pos = carry + block_excl_scan(i < ne ? count[i] : 0, &total);
+    if (i < ne) count[i] = pos;
+    carry += total;
   }
   __syncthreads();
   for (int i = threadIdx.x; i < ne; i += kRgStageThreads) {
-    int rank = 0;
-    for (int j = 0; j < ne; ++j) rank += first[j] < first[i] || (first[j] == first[i] && j < i);
+    const int f = first[i];
+    int rank = count[f];
+    for (int j = f; j < i; ++j) rank += first[j] == f;
     out[start + rank] = order[start + i];
   }
 }
@@ -776,7 +792,7 @@ static int region_plan_build(int32_t set_size, int32_t part_size, int32_t region
                           cudaMemcpyHostToDevice, s));
 
   if (even && nblocks > 0) {
-    const int gsmem = 2 * part_size * (int)sizeof(int32_t);
+    const int gsmem = 3 * part_size * (int)sizeof(int32_t);
     int32_t *grouped = nullptr;
     RG_TRY(alloc((void **)&grouped, sizeof(int32_t) * n, true));
     RG_CUDA(cudaFuncSetAttribute(rg_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gsmem));
@@ -848,33 +864,42 @@ static int region_plan_build(int32_t set_size, int32_t part_size, int32_t region
         mask_words += P->max_count[q];
         inc_rows += stage_arity[q];
       }
-    const int64_t cwords = mask_words + (int64_t)part_size * inc_rows + 2LL * part_size + 1;
-    if (cwords * 4 > smem_optin())
-      return fail(set_error(OP2B_ERR_ARG, "region plan: colouring needs %lld bytes of shared memory",
-                            (long long)(cwords * 4)));
-    const int csmem = (int)sizeof(uint32_t) * (int)std::max<int64_t>(cwords, 1);
-    RG_CUDA(cudaFuncSetAttribute(rg_color_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
-    int32_t *newpos = nullptr, *order2 = nullptr;
-    int16_t *loc2 = nullptr;
-    RG_TRY(alloc((void **)&newpos, sizeof(int32_t) * n, true));
-    RG_TRY(alloc((void **)&order2, sizeof(int32_t) * n, true));
-    RG_TRY(alloc((void **)&loc2, sizeof(int16_t) * (size_t)loc_rows * n, true));
-    rg_color_kernel<<<nblocks, 32, csmem, s>>>(d_st, d_inc, nstage, n, inc_rows, part_size, P->boff,
-                                                P->tcnt, P->loc, P->thrcol, P->nthrcol, newpos);
-    RG_CUDA(cudaGetLastError());
-    rg_permute_kernel<<<grid, kRgThreads, 0, s>>>(n, loc_rows, newpos, P->order, P->loc, order2, loc2);
-    RG_CUDA(cudaGetLastError());
-    // the permuted arrays replace the originals, which become temporaries
-    temps.erase(std::remove(temps.begin(), temps.end(), (void *)order2), temps.end());
-    temps.erase(std::remove(temps.begin(), temps.end(), (void *)loc2), temps.end());
-    temps.push_back(P->order);
-    temps.push_back(P->loc);
-    P->order = order2;
-    P->loc = loc2;
-    std::vector<int32_t> h_nc(nblocks);
-    RG_CUDA(cudaMemcpyAsync(h_nc.data(), P->nthrcol, sizeof(int32_t) * nblocks, cudaMemcpyDeviceToHost, s));
-    RG_CUDA(cudaStreamSynchronize(s));
-    for (int b = 0; b < nblocks; ++b) P->max_nthrcol = std::max(P->max_nthrcol, h_nc[b]);
+    if (inc_rows == 0) {
+      // nothing to keep apart: one colour, the order as it is
+      const std::vector<int32_t> one(nblocks, 1);
+      RG_CUDA(cudaMemsetAsync(P->thrcol, 0, sizeof(int32_t) * n, s));
+      RG_CUDA(cudaMemcpyAsync(P->nthrcol, one.data(), sizeof(int32_t) * nblocks, cudaMemcpyHostToDevice, s));
+      RG_CUDA(cudaStreamSynchronize(s));
+      P->max_nthrcol = 1;
+    } else {
+      const int64_t cwords = mask_words + (int64_t)part_size * inc_rows + 2LL * part_size + 1;
+      if (cwords * 4 > smem_optin())
+        return fail(set_error(OP2B_ERR_ARG, "region plan: colouring needs %lld bytes of shared memory",
+                              (long long)(cwords * 4)));
+      const int csmem = (int)sizeof(uint32_t) * (int)std::max<int64_t>(cwords, 1);
+      RG_CUDA(cudaFuncSetAttribute(rg_color_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, csmem));
+      int32_t *newpos = nullptr, *order2 = nullptr;
+      int16_t *loc2 = nullptr;
+      RG_TRY(alloc((void **)&newpos, sizeof(int32_t) * n, true));
+      RG_TRY(alloc((void **)&order2, sizeof(int32_t) * n, true));
+      RG_TRY(alloc((void **)&loc2, sizeof(int16_t) * (size_t)loc_rows * n, true));
+      rg_color_kernel<<<nblocks, 32, csmem, s>>>(d_st, d_inc, nstage, n, inc_rows, part_size, P->boff,
+                                                  P->tcnt, P->loc, P->thrcol, P->nthrcol, newpos);
+      RG_CUDA(cudaGetLastError());
+      rg_permute_kernel<<<grid, kRgThreads, 0, s>>>(n, loc_rows, newpos, P->order, P->loc, order2, loc2);
+      RG_CUDA(cudaGetLastError());
+      // the permuted arrays replace the originals, which become temporaries
+      temps.erase(std::remove(temps.begin(), temps.end(), (void *)order2), temps.end());
+      temps.erase(std::remove(temps.begin(), temps.end(), (void *)loc2), temps.end());
+      temps.push_back(P->order);
+      temps.push_back(P->loc);
+      P->order = order2;
+      P->loc = loc2;
+      std::vector<int32_t> h_nc(nblocks);
+      RG_CUDA(cudaMemcpyAsync(h_nc.data(), P->nthrcol, sizeof(int32_t) * nblocks, cudaMemcpyDeviceToHost, s));
+      RG_CUDA(cudaStreamSynchronize(s));
+      for (int b = 0; b < nblocks; ++b) P->max_nthrcol = std::max(P->max_nthrcol, h_nc[b]);
+    }
   } else {
     RG_TRY(alloc((void **)&P->tlist, 16, false));
     RG_CUDA(cudaMemsetAsync(P->toff, 0, sizeof(int32_t) * ((size_t)nblocks * nstage + 1), s));
