@@ -170,22 +170,15 @@ def pinned_empty(shape, dtype):
 
 
 def copies(arrays):
-    """Fresh copies of a dict of numpy arrays.  Most of such a copy is the page
+    """Fresh copies of a dict of numpy arrays.  Most of a large copy is the page
     faults of the new memory, which several threads take at once
     (op2b_host_copy); a thread that waits in it does not hold the interpreter."""
-    out, dst, src, nbytes = {}, [], [], []
-    for k, v in arrays.items():
-        if type(v) is not np.ndarray or v.dtype.hasobject or not v.flags.c_contiguous:
-            out[k] = np.array(v)
-            continue
-        out[k] = a = np.empty(v.shape, v.dtype)
-        dst.append(a.ctypes.data)
-        src.append(v.ctypes.data)
-        nbytes.append(v.nbytes)
-    n = len(dst)
-    if n:
-        u64s = C.c_uint64 * n
-        call("op2b_host_copy", n, u64s(*dst), u64s(*src), u64s(*nbytes))
+    plain = {k: v for k, v in arrays.items()
+             if type(v) is np.ndarray and not v.dtype.hasobject and v.flags.c_contiguous}
+    out = {k: np.empty(v.shape, v.dtype) if k in plain else np.array(v) for k, v in arrays.items()}
+    u64s = C.c_uint64 * len(plain)
+    call("op2b_host_copy", len(plain), u64s(*[out[k].ctypes.data for k in plain]),
+         u64s(*[v.ctypes.data for v in plain.values()]), u64s(*[v.nbytes for v in plain.values()]))
     return out
 
 

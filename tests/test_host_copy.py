@@ -30,3 +30,26 @@ def test_copies_of_other_layouts():
     np.testing.assert_array_equal(got["s"], a[:, ::3])
     np.testing.assert_array_equal(got["r"], a)
     assert got["r"].flags.writeable and got["x"] == 4.0
+
+
+def test_copies_from_several_threads():
+    """Callers at once, each with its own arrays (more pieces than threads)."""
+    import threading
+    from pyop2_b200 import b200
+    _lib.load()
+    rng = np.random.default_rng(9)
+    src = [{"a": rng.integers(0, 256, (2 << 20) + 13 * k, dtype=np.uint8), "b": np.arange(5.0) + k}
+           for k in range(6)]
+    bad = []
+
+    def run(mine):
+        for _ in range(8):
+            got = b200.copies(mine)
+            if not all(np.array_equal(got[k], mine[k]) for k in mine):
+                bad.append(mine)
+    threads = [threading.Thread(target=run, args=(s,)) for s in src]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
