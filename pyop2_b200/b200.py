@@ -2639,6 +2639,8 @@ def _rows_before_capture():
     for bl in list(ParLoop._bound_cache.values()):
         if bl._rows_later and bl._last_run > since:
             bl._to_rows(bl._args)
+            # now, not as copies in the graph: the new form's module has not run
+            _sync_consts(bl.module, bl.consts)
 
 
 class capture(object):

@@ -164,3 +164,35 @@ def test_row_blocks_are_built_when_a_loop_keeps_running(op2, monkeypatch):
     assert mode("p1_stiff", P.elements) == ["rowblk"]
     g.launch()
     np.testing.assert_allclose(P.stiff.array, one, rtol=1e-14, atol=1e-16)
+
+
+def test_consts_of_a_form_built_for_a_capture(backend, monkeypatch):
+    """A loop bound again as row blocks before a capture has its Consts at once: a
+    run of the loop is right although the graph was never launched."""
+    from pyop2_b200 import b200, op2
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", (0, 0))
+    scale = op2.Const(1, 2.5, "rowblk_scale", np.float64)
+    try:
+        coords, elem = meshes.rect_p1(9, 7, 1)
+        P = fem.build_p1(op2, 0, coords=coords, elem=elem)
+        k = op2.Kernel("void scaled(double A[1][1], double **x, int i, int j) "
+                       "{ A[0][0] += rowblk_scale * (1 + i + 2 * j); }", "scaled")
+        m = P.elem_node
+
+        def loop():
+            P.mat.zero()
+            op2.par_loop(k, P.elements(3, 3), P.mat((m[op2.i[0]], m[op2.i[1]]), op2.INC),
+                         P.coords(P.elem_vnode, op2.READ))
+        loop()
+        want = P.mat.array.copy()
+        assert abs(want).max() > 0
+        with b200.capture() as g:
+            loop()
+        forms = [bl.spec.mode for bl in b200.ParLoop._bound_cache.values() if bl.spec.kernel_name == "scaled"]
+        assert forms == ["rowblk"]
+        loop()
+        np.testing.assert_allclose(P.mat.array, want, rtol=1e-14)
+        g.launch()
+        np.testing.assert_allclose(P.mat.array, want, rtol=1e-14)
+    finally:
+        scale.remove_from_namespace()
