@@ -1210,13 +1210,13 @@ _ROWBLK_THREADS = 128
 _ROWBLK_BYTES = 18 << 10
 
 
-# contributions a launch adds, below which the form makes no difference worth
-# its tables, for local blocks below 6 x 6 and from there on.  In a graph with
-# the memsets and P1's RHS: P1 256 x 256 (1.2 million) 15.7 us against 14.4 with
-# structured numbering and 14.5 against 17.4 permuted, P1 320 x 320 (1.8 million)
-# 20.6 against 22.7; P2 128 x 128 (1.2 million) 16.5 against 22.7, 64 x 64 (0.3
-# million) 10.4 against 11.9
-_ROWBLK_MIN = (3 << 19, 1 << 20)
+# contributions a launch adds, below which the form makes too little difference
+# for its tables (0.4 ms to build).  In a graph with the memsets and P1's RHS,
+# element form against row blocks: P1 256 x 256 (1.2 million) 14.3 us against 13.0
+# with structured numbering and 17.8 against 14.6 permuted, 222 x 222 (0.9 million) 12.4 against 12.4 and 14.5 against 14.5; P2
+# 128 x 128 (1.2 million) 20.6 against 16.5, 91 x 91 (0.6 million) 14.5 against
+# 12.4, 64 x 64 (0.3 million) 11.1 against 9.8
+_ROWBLK_MIN = 1 << 20
 
 # runs of a bound loop before its row blocks are built: the build takes what 30
 # (P2) to 80 (P1) runs then save, and the element form needs only the slot table,
@@ -1728,7 +1728,7 @@ class _BoundLoop(object):
         self._rows_later = bool(
             w is not None and nelem is None and inc_mode is None and not _partitioned(iterset)
             and (spec.mode == "lma" or (spec.mode == "atomic" and _default_mat_form()))
-            and iterset.size * w.arity * w.carity >= _ROWBLK_MIN[w.arity * w.carity >= 36]
+            and iterset.size * w.arity * w.carity >= _ROWBLK_MIN
             and codegen.rowblk_capable(spec))
         if self._rows_later and (rows or spec.mode == "lma"):
             self._rows_later = False

@@ -18,7 +18,7 @@ def op2(backend, monkeypatch):
     """Every assembly runs as row blocks from its first run."""
     from pyop2_b200 import b200, op2
     monkeypatch.setattr(b200, "_ROWBLK_RUNS", 0)
-    monkeypatch.setattr(b200, "_ROWBLK_MIN", (0, 0))
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
     return op2
 
 
@@ -142,7 +142,7 @@ def test_row_blocks_are_built_when_a_loop_keeps_running(op2, monkeypatch):
     capture of a loop that ran just before; small loops keep their form."""
     from pyop2_b200 import b200
     monkeypatch.setattr(b200, "_ROWBLK_RUNS", 3)
-    monkeypatch.setattr(b200, "_ROWBLK_MIN", (9 * 2 * 12 * 11, 0))
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 9 * 2 * 12 * 11)
     coords, elem = meshes.rect_p1(12, 11, 1)
     small_c, small_e = meshes.rect_p1(5, 4, 1)
     P = fem.build_p1(op2, 0, coords=coords, elem=elem, stiffness=True)
@@ -170,7 +170,7 @@ def test_consts_of_a_form_built_for_a_capture(backend, monkeypatch):
     """A loop bound again as row blocks before a capture has its Consts at once: a
     run of the loop is right although the graph was never launched."""
     from pyop2_b200 import b200, op2
-    monkeypatch.setattr(b200, "_ROWBLK_MIN", (0, 0))
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
     scale = op2.Const(1, 2.5, "rowblk_scale", np.float64)
     try:
         coords, elem = meshes.rect_p1(9, 7, 1)
