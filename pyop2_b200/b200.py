@@ -1213,9 +1213,10 @@ _ROWBLK_BYTES = 18 << 10
 # contributions a launch adds, below which the form makes too little difference
 # for its tables (0.4 ms to build).  In a graph with the memsets and P1's RHS,
 # element form against row blocks: P1 256 x 256 (1.2 million) 14.3 us against 13.0
-# with structured numbering and 17.8 against 14.6 permuted, 222 x 222 (0.9 million) 12.4 against 12.4 and 14.5 against 14.5; P2
-# 128 x 128 (1.2 million) 20.6 against 16.5, 91 x 91 (0.6 million) 14.5 against
-# 12.4, 64 x 64 (0.3 million) 11.1 against 9.8
+# with structured numbering and 17.8 against 14.6 permuted, 222 x 222 (0.9 million)
+# 12.4 against 12.4 and 14.5 against 14.5; P2 128 x 128 (1.2 million) 20.6 against
+# 16.5, 91 x 91 (0.6 million) 14.5 against 12.4, 64 x 64 (0.3 million) 11.1
+# against 9.8
 _ROWBLK_MIN = 1 << 20
 
 # runs of a bound loop before its row blocks are built: the build takes what 30
