@@ -867,6 +867,8 @@ class DevicePlan(object):
 
 _REGION_ARRAYS = ("order", "boff", "tlist", "toff", "tcnt", "loc", "thrcol", "nthrcol")
 _REGION_CACHE = {}
+# (element, Map row) pairs of a block that op2b_region_plan_build takes
+_REGION_KEYS = 16384
 
 
 class RegionPlan(object):
@@ -1546,7 +1548,7 @@ def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=Non
         spec.mode = "gather"
         R = _region_layout(specs, maps)
         ps = int(cfg.cfg['partition_size']) or 384
-        R["part_size"] = max(1, min(ps, 16384 // max(R["stage_arity"])))
+        R["part_size"] = max(1, min(ps, _REGION_KEYS // max(R["stage_arity"])))
         gather_region = R
         indirect = False
     elif (indirect and req in ('staged', 'gather') and codegen.staged_capable(spec)
@@ -1557,10 +1559,12 @@ def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=Non
             spec.block_size = bs = int(cfg.cfg['staged_block_size'])
         # blocks of at most part_size elements; the stub runs ept passes of bs
         ps = int(cfg.cfg['partition_size']) or 384
-        ps = max(1, min(ps, 16384 // max(R["stage_arity"])))
+        # the builder takes at most _REGION_KEYS (element, Map row) pairs a block
+        most = max(1, _REGION_KEYS // max(R["stage_arity"]))
+        ps = min(ps, most)
         if (int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
                 and not cfg.cfg['staged_tl_regs']):
-            part = codegen.staged_sums(spec, min(ps, int(cfg.cfg['partition_size'])))
+            part = codegen.staged_sums(spec, int(cfg.cfg['partition_size']), most)
             if part:
                 R["sums"], ps = True, part
                 R["ids"] = any(s.kind == "direct" for s in specs)

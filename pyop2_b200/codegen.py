@@ -772,11 +772,12 @@ def staged_smem(spec, max_count, max_elems=0, max_packet=0):
 _SUMS_PARTS = ((256, 24 << 10), (128, 96 << 10))
 
 
-def staged_sums(spec, part_size=0):
+def staged_sums(spec, part_size, most):
     """Elements per block with which a staged loop stores its contributions and
-    sums them per target (``part_size`` if given), or 0 where it adds them colour
-    by colour: every INC (Dat, staged Map) pair has to be incremented through each
-    row of the Map once, and a block's contributions to fit."""
+    sums them per target (``part_size`` if not 0, at most ``most``), or 0 where it
+    adds them colour by colour: every INC (Dat, staged Map) pair has to be
+    incremented through each row of the Map once, and a block's contributions to
+    fit."""
     R = spec.region
     rows = {}
     for a in spec.args:
@@ -784,13 +785,14 @@ def staged_sums(spec, part_size=0):
             st = R["map_stage"][a.mslot]
             rows.setdefault((a.slot, st), []).extend(
                 [a.idx] if a.kind == "ind" else range(a.arity if a.kind == "vec" else a.ext))
+    part_size = min(part_size, most)
     if (len(R["stage_arity"]) > 4 or part_size > 1024
             or any(sorted(r) != list(range(R["stage_arity"][st])) for (_, st), r in rows.items())):
         return 0
     one = sum(R["stage_arity"][st] * c * _CSIZE[t] for _, st, t, c in R["inc_pairs"])
     if part_size:
         return part_size if part_size * one <= _SUMS_PARTS[-1][1] else 0
-    return next((n for n, room in _SUMS_PARTS if n * one <= room), 0)
+    return next((n for n, room in _SUMS_PARTS if n <= most and n * one <= room), 0)
 
 
 def _sums_chunk(ctype, cdim):
