@@ -1562,7 +1562,8 @@ def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=Non
         # the builder takes at most _REGION_KEYS (element, Map row) pairs a block
         most = max(1, _REGION_KEYS // max(R["stage_arity"]))
         ps = min(ps, most)
-        if (int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
+        # (whole warps add up the targets' rows: op2b_row_share)
+        if (bs % 32 == 0 and int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
                 and not cfg.cfg['staged_tl_regs']):
             part = codegen.staged_sums(spec, int(cfg.cfg['partition_size']), most)
             if part:

@@ -42,7 +42,8 @@ keys of the B200 backend:
   size, whose default in the staged form is 384; where contributions are
   summed per target instead of colour by colour, 5/4 of the 256 or 128
   elements of a block);
-* ``staged_block_size``: threads per CTA of the staged form's stubs;
+* ``staged_block_size``: threads per CTA of the staged form's stubs (a size that is
+  not a multiple of 32 selects the one that adds colour by colour);
 * ``staged_tl_regs``: (this and the next two select the staged form that adds
   colour by colour, which they tune) the staged stubs load their block's target ids into
   registers once (with the element rows) and reuse them for the row copies

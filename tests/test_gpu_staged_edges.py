@@ -44,3 +44,15 @@ def test_maps_with_many_rows(op2, inc, read, sums):
     got = run(op2, 2003, inc, read)
     assert bound().spec.mode == "staged" and bool(bound().spec.region.get("sums")) == sums
     np.testing.assert_array_equal(got, run(seq, 2003, inc, read))
+
+
+@pytest.mark.parametrize("threads", [32, 96, 100, 128, 130])
+@pytest.mark.parametrize("cdim", [1, 3, 4])
+def test_cta_sizes(op2, threads, cdim):
+    """CTAs that are not whole warps run the colour form (the summing form's
+    shuffles name every lane)."""
+    cfg.configure(staged_block_size=threads)
+    got = run(op2, 1501, 2, 3, cdim)
+    assert bound().spec.mode == "staged"
+    assert bool(bound().spec.region.get("sums")) == (threads % 32 == 0)
+    np.testing.assert_array_equal(got, run(seq, 1501, 2, 3, cdim))

@@ -49,3 +49,13 @@ def test_blocks_of_maps_with_many_rows(op2, inc, read, dtype, elems, part):
     else:
         assert bool(R.get("sums")) == (elems > 0)
         assert R["part_size"] == (elems or min(384, most))
+
+
+@pytest.mark.parametrize("threads,sums", [(32, True), (96, True), (128, True), (256, True), (100, False),
+                                          (1, False), (129, False)])
+def test_cta_sizes_of_the_summing_form(op2, threads, sums):
+    """Its sums are shared by whole warps: other CTA sizes keep the colour form."""
+    cfg.configure(staged_block_size=threads)
+    spec = loop_spec(op2, 2, 3)
+    assert spec.mode == "staged" and spec.block_size == threads
+    assert bool(spec.region.get("sums")) == sums
