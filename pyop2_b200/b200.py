@@ -1387,10 +1387,11 @@ def mat_slot_values(specs, maps, mats, rel=False):
 
 
 def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=None,
-              inc_mode=None, min_blocks=None, size=None):
+              inc_mode=None, min_blocks=None, size=None, sums=True):
     """Static description of a par_loop: the LoopSpec of its stub plus the
     unique Dats/Maps/Mats/Globals, the INC staging pairs and the plan race
-    groups.  Touches no device memory (used to generate and test stubs)."""
+    groups.  ``sums``: a staged loop may take the summing form.  Touches no
+    device memory (used to generate and test stubs)."""
     it = loop.it_space
     iterset = it.iterset
     nsz = iterset.size if size is None else int(size)
@@ -1563,7 +1564,7 @@ def loop_spec(loop, block_size=None, fmad=None, owner_mode=None, mat_nnz_max=Non
         most = max(1, _REGION_KEYS // max(R["stage_arity"]))
         ps = min(ps, most)
         # (whole warps add up the targets' rows: op2b_row_share)
-        if (bs % 32 == 0 and int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
+        if (sums and bs % 32 == 0 and int(cfg.cfg['staged_pair']) != 2 and not cfg.cfg['staged_bank_slots']
                 and not cfg.cfg['staged_tl_regs']):
             part = codegen.staged_sums(spec, int(cfg.cfg['partition_size']), most)
             if part:
@@ -1706,18 +1707,37 @@ def _default_mat_form():
 
 class _StagedTooLarge(Exception):
     """The staged form of a loop needs more shared memory per CTA than the
-    device has: the loop is bound in the atomic form instead."""
+    device has.  ``sums``: the summing form does, which holds two packets and the
+    contributions beside the rows; the form that adds colour by colour may fit."""
+
+    def __init__(self, sums):
+        Exception.__init__(self)
+        self.sums = sums
+
+
+def _bind_fitting(loop, nelem=None):
+    """The loop bound in the staged form that fits, or as configured where it is
+    not staged; None if neither staged form fits."""
+    try:
+        return _BoundLoop(loop, nelem=nelem)
+    except _StagedTooLarge as e:
+        if not e.sums:
+            return None
+    try:
+        return _BoundLoop(loop, nelem=nelem, sums=False)
+    except _StagedTooLarge:
+        return None
 
 
 class _BoundLoop(object):
     """Everything about a par_loop that does not change between calls with
     the same objects: generated stub, plan, parameter block."""
 
-    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None, rows=False):
+    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None, rows=False, sums=True):
         # nelem: bind to the set's first nelem elements only (the core of a
         # partitioned set, run in the staged form); rows: in the row block form
-        # if it runs the loop
-        info = loop_spec(loop, inc_mode=inc_mode, owner_mode=owner_mode, size=nelem)
+        # if it runs the loop; sums: the summing staged form may be taken
+        info = loop_spec(loop, inc_mode=inc_mode, owner_mode=owner_mode, size=nelem, sums=sums)
         spec = info['spec']
         specs = info['specs']
         dats, maps, mats, gbls = info['dats'], info['maps'], info['mats'], info['gbls']
@@ -1859,17 +1879,17 @@ class _BoundLoop(object):
             self.region_plan = rp
             for name in _REGION_ARRAYS:
                 vals["rg_" + name] = rp.dptr[name]
-            sums = ()
+            room = ()
             if spec.region.get("sums"):
-                vals["rg_dir"], vals["rg_pkt"], *sums = rp.packets(spec.region["inc_stages"],
+                vals["rg_dir"], vals["rg_pkt"], *room = rp.packets(spec.region["inc_stages"],
                                                                    spec.region["ids"])
-                vals["rg_blocks"], self.room = rp.nblocks, sums[1]
-            self.launch_smem = codegen.staged_smem(spec, rp.max_count, *sums)
+                vals["rg_blocks"], self.room = rp.nblocks, room[1]
+            self.launch_smem = codegen.staged_smem(spec, rp.max_count, *room)
             if self.launch_smem > _state['smem_optin']:
-                raise _StagedTooLarge()
+                raise _StagedTooLarge(bool(room))
             self.module.ensure_smem(self.launch_smem)
             self.grid = rp.nblocks
-            if sums:
+            if room:
                 occ = max(1, self.module.occupancy(self.module.fn, spec.block_size, self.launch_smem))
                 self.grid = min(rp.nblocks, occ * _state['sm_count'])
             self.max_grid = max(1, self.grid)
@@ -2418,17 +2438,11 @@ def _bind(loop, iterset):
         if bl.spec.mode == "atomic" and core > 0 and cfg.cfg['inc_mode'] in ('staged', 'gather'):
             # the core (most of a rank's elements) in the staged form over a
             # locality partition of its own; the other ranges stay atomic
-            try:
-                cb = _BoundLoop(loop, nelem=core)
-            except _StagedTooLarge:
-                cb = None
+            cb = _bind_fitting(loop, nelem=core)
             if cb is not None and cb.spec.mode == "staged":
                 bl.core_loop = cb
         return bl
-    try:
-        return _BoundLoop(loop)
-    except _StagedTooLarge:
-        return _BoundLoop(loop, inc_mode='atomic')
+    return _bind_fitting(loop) or _BoundLoop(loop, inc_mode='atomic')
 
 
 class ParLoop(base.ParLoop):

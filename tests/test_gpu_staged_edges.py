@@ -16,11 +16,11 @@ def op2(backend):
     return op2
 
 
-def run(api, n, inc, read, cdim=1, rdim=1):
+def run(api, n, inc, read, cdim=1, rdim=1, nx=None):
     """y += sums of rows of x, through Maps of arity ``inc`` and ``read``; whole
     numbers, exact in any order."""
     rng = np.random.default_rng(n + inc + read)
-    ny, nx = n // 3 + inc, n // 2 + read
+    ny, nx = n // 3 + inc, nx or n // 2 + read
     el, nd, nr = api.Set(n, 1, "el"), api.Set(ny, cdim, "nd"), api.Set(nx, rdim, "nr")
     m = api.Map(el, nd, inc, rng.integers(0, ny, (n, inc)).astype(np.int32), "m")
     r = api.Map(el, nr, read, rng.integers(0, nx, (n, read)).astype(np.int32), "r")
@@ -56,3 +56,13 @@ def test_cta_sizes(op2, threads, cdim):
     assert bound().spec.mode == "staged"
     assert bool(bound().spec.region.get("sums")) == (threads % 32 == 0)
     np.testing.assert_array_equal(got, run(seq, 1501, 2, 3, cdim))
+
+
+@pytest.mark.parametrize("read,rdim,mode", [(100, 1, "staged"), (120, 1, "staged"), (120, 2, "atomic")])
+def test_rows_that_fill_the_shared_memory(op2, read, rdim, mode):
+    """Nearly every element of a block names rows of its own.  What the summing
+    form, with its packets, has no room for still runs colour by colour; the
+    atomic form takes what neither can."""
+    got = run(op2, 2003, 2, read, 1, rdim, nx=400000)
+    assert bound().spec.mode == mode and not (bound().spec.region or {}).get("sums")
+    np.testing.assert_array_equal(got, run(seq, 2003, 2, read, 1, rdim, nx=400000))
