@@ -461,29 +461,32 @@ struct DotScratch {
   DotResult *result = nullptr;
   unsigned long long ticket = 0;
 
-  int ready(int most) {
+  // The counter is cleared on the call's stream and waited for, once per thread
+  // and device: later calls may come on any stream.
+  int ready(int most, cudaStream_t s) {
     int dev = 0;
     OP2B_CUDA(cudaGetDevice(&dev));
     if (dev == device) return OP2B_OK;
     release();
-    double *p = nullptr;
-    OP2B_CUDA(cudaMalloc((void **)&p, sizeof(double) * (most + 2)));
-    cudaError_t e = cudaMemset(p, 0, sizeof(double) * (most + 2));
+    const size_t bytes = sizeof(double) * (most + 2);
+    cudaError_t e = cudaMalloc((void **)&part, bytes);
     if (e == cudaSuccess) e = cudaHostAlloc((void **)&result, sizeof(DotResult), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, bytes, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
-      cudaFree(p);
+      release();
       return check_cuda(e, "op2b_vec_dot scratch");
     }
     result->ticket = ticket = 0;
-    part = p;
-    counter = reinterpret_cast<unsigned *>(p + most);
+    counter = reinterpret_cast<unsigned *>(part + most);
     device = dev;
     return OP2B_OK;
   }
   void release() {
-    if (device < 0) return;
-    cudaFree(part);
-    cudaFreeHost(result);
+    if (part) cudaFree(part);
+    if (result) cudaFreeHost(result);
+    part = nullptr;
+    result = nullptr;
     device = -1;
   }
   ~DotScratch() { release(); }
@@ -546,7 +549,7 @@ int op2b_vec_dot(uint64_t x, uint64_t y, int64_t n, double *result, uint64_t str
   cudaStream_t s = stream_of(stream);
   const int most = sm_count() * 4;
   DotScratch &w = t_dot;
-  int rc = w.ready(most);
+  int rc = w.ready(most, s);
   if (rc) return rc;
   const int W = (x | y) % 16 ? 1 : 2;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n / W + kLinBlock - 1) / kLinBlock, most));
@@ -565,6 +568,10 @@ int op2b_vec_dot(uint64_t x, uint64_t y, int64_t n, double *result, uint64_t str
   bool in = false;
   for (int spin = 0; spin < 100000 && !in; ++spin) in = *seen == ticket;
   if (!in) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && !in && *seen != ticket) {
+    w.release();       // no CTA saw itself as the last one: never a value of an earlier call
+    return set_error(OP2B_ERR_CUDA, "op2b_vec_dot: the kernel left no result");
+  }
   if (e == cudaSuccess) *result = *(const volatile double *)&w.result->value;
   return check_cuda(e, "op2b_vec_dot");
 }

@@ -1,0 +1,68 @@
+"""Calls from several host threads: what each keeps for itself is ready in time."""
+
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def in_threads(n, work):
+    """work(k) in n threads at once; their results."""
+    got, start = [None] * n, threading.Barrier(n)
+
+    def run(k):
+        start.wait()
+        try:
+            got[k] = work(k)
+        except Exception as e:      # shown by the comparison
+            got[k] = e
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    return got
+
+
+@pytest.mark.parametrize("size", [1, 257, 300001])
+def test_first_dot_of_a_thread(backend, size):
+    """A thread's first dot product, while the stream is busy: whole numbers, so
+    exact in any order; the scratch is cleared before the kernel counts in it."""
+    from pyop2_b200 import b200
+    from pyop2_b200._lib import call
+    x = np.random.default_rng(size).integers(-9, 10, size).astype(np.float64)
+    d = b200._upload(x)
+    busy = b200.DeviceBuffer(1 << 28)
+    want = float(x @ x)
+
+    def dots(k):
+        out = []
+        for _ in range(3):
+            r = C.c_double(-1.0)
+            busy.memset(k)
+            call("op2b_vec_dot", d.ptr, d.ptr, size, C.byref(r), 0)
+            out.append(r.value)
+        return out
+    for _ in range(5):
+        assert in_threads(6, dots) == [[want] * 3] * 6
+
+
+def test_small_downloads_of_several_threads(backend):
+    """Downloads of at most 256 bytes land in memory of the calling thread."""
+    from pyop2_b200 import b200
+    rng = np.random.default_rng(2)
+    want = [rng.integers(0, 256, 200, dtype=np.uint8) for _ in range(6)]
+    bufs = [b200._upload(w) for w in want]
+
+    def down(k):
+        out = np.zeros(200, np.uint8)
+        for _ in range(50):
+            out[:] = 0
+            bufs[k].to_host(out)
+            if not np.array_equal(out, want[k]):
+                return "wrong"
+        return "right"
+    assert in_threads(6, down) == ["right"] * 6
