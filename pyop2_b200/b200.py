@@ -1747,6 +1747,8 @@ class _BoundLoop(object):
         self.row_blocks = None
         self.room = 0       # 16-byte units of a packet (row blocks, summing staged form)
         self._runs, self._last_run = 0, -_ROWBLK_RECENT
+        self.key = None     # in ParLoop._bound_cache
+        self._written = []
         # Mat assembly by the owners of the rows (see codegen._rowblk_body): at
         # once in place of the two-phase form, whose own tables cost as much to
         # build; else when the loop has run often enough (see run)
@@ -2048,21 +2050,31 @@ class _BoundLoop(object):
         n = self.nelem if rng is None else rng[1] - rng[0]
         trace.append((pre, _capture_tail(), self.accesses + gbl, n))
 
-    def _to_rows(self, args):
-        """Bind again in the row block form (the element form where that
-        does not run the loop)."""
-        kernel, it_space = self._again
-        trace_runs = self._runs
-        _BoundLoop.__init__(self, _Loop(kernel, it_space, args), rows=True)
-        self._buf, self._runs = None, trace_runs
+    def _in_rows(self, args):
+        """The loop bound in the row block form, which takes this bound loop's
+        place in the cache; this one where that form does not run the loop.  It
+        stays as it is, since another thread may be running it."""
+        self._rows_later, self._args = False, None
+        loop = _Loop(self._again[0], self._again[1], args)
+        new = _BoundLoop(loop, rows=True)
+        if new.row_blocks is None:
+            return self
+        new.key = self.key
+        new._prepare(loop)
+        if ParLoop._bound_cache.get(self.key) is self:
+            ParLoop._bound_cache[self.key] = new
+        return new
 
     def _run(self, loop, rng=None):
         _runs[0] += 1
         if self._rows_later:
             self._runs += 1
             self._last_run, self._args = _runs[0], loop.args
-            if self._runs > _ROWBLK_RUNS and not _state.get('capturing'):
-                self._to_rows(self._args)
+            if self._runs > _ROWBLK_RUNS and rng is None and not _state.get('capturing'):
+                form = self._in_rows(loop.args)
+                if form is not self:
+                    form._run(loop)
+                    return
         if getattr(self, "_buf", None) is None:
             self._prepare(loop)
         for d in self.dats:
@@ -2457,6 +2469,7 @@ class ParLoop(base.ParLoop):
         bl = ParLoop._bound_cache.get(key)
         if bl is None or not bl.matches(self):
             bl = _bind(self, self.it_space.iterset)
+            bl.key = key
             ParLoop._bound_cache[key] = bl
         return bl
 
@@ -2658,9 +2671,9 @@ def _rows_before_capture():
     since = _runs[0] - _ROWBLK_RECENT
     for bl in list(ParLoop._bound_cache.values()):
         if bl._rows_later and bl._last_run > since:
-            bl._to_rows(bl._args)
+            new = bl._in_rows(bl._args)
             # now, not as copies in the graph: the new form's module has not run
-            _sync_consts(bl.module, bl.consts)
+            _sync_consts(new.module, new.consts)
 
 
 class capture(object):

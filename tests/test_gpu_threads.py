@@ -66,3 +66,37 @@ def test_small_downloads_of_several_threads(backend):
                 return "wrong"
         return "right"
     assert in_threads(6, down) == ["right"] * 6
+
+
+def test_a_loop_changes_form_while_threads_run_it(backend, monkeypatch):
+    """Threads repeat one assembly; one of them binds it as row blocks while the
+    others are in the element form.  Whole numbers: exact in any order."""
+    from pyop2_b200 import b200, op2
+    from pyop2_b200.workloads import meshes
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
+    coords, elem = meshes.rect_p1(40, 31, 2)
+    n, nodes = len(elem), len(coords)
+    el, nd = op2.Set(n, 1, "el"), op2.Set(nodes, 1, "nd")
+    m = op2.Map(el, nd, 3, elem, "m")
+    k = op2.Kernel("void threads(double A[1][1], double *w, int i, int j) { A[0][0] += w[0] * (1 + 3 * i + j); }",
+                   "threads")
+    w = op2.Dat(el, np.random.default_rng(1).integers(1, 9, n).astype(np.float64), np.float64, "w")
+
+    def assemble(mat):
+        op2.par_loop(k, el(3, 3), mat((m[op2.i[0]], m[op2.i[1]]), op2.INC), w(op2.IdentityMap, op2.READ))
+    sp = op2.Sparsity((m, m), "s")
+    one = op2.Mat(sp, np.float64, "one")
+    assemble(one)
+    for _ in range(4):
+        monkeypatch.setattr(b200, "_ROWBLK_RUNS", 8)
+        mat = op2.Mat(sp, np.float64, "mat")
+        assemble(mat)          # bound
+
+        def work(_):
+            for _ in range(10):
+                assemble(mat)
+            return True
+        assert in_threads(4, work) == [True] * 4
+        forms = [b.spec.mode for b in b200.ParLoop._bound_cache.values() if b.mats == [mat]]
+        assert forms == ["rowblk"]
+        np.testing.assert_array_equal(mat.array, 41 * one.array)
