@@ -22,6 +22,7 @@ import ctypes as C
 import hashlib
 import os
 import struct
+import threading
 import weakref
 
 import numpy as np
@@ -640,6 +641,12 @@ class Sparsity(base.Sparsity):
             pass
 
 
+# Held while work that writes a Mat is issued and what is known of its values
+# changes with it: another thread's loop, issued between the two, would take a Mat
+# for zero that no longer is (or the other way round)
+_MAT_LOCK = threading.RLock()
+
+
 class Mat(DeviceDataMixin, base.Mat):
     """Device CSR values on a Sparsity."""
 
@@ -682,11 +689,13 @@ class Mat(DeviceDataMixin, base.Mat):
         return ret
 
     def zero(self):
-        self._device_values().memset(0)
-        graph = _state.get('capturing')
-        self._zeroed = graph if graph else True
-        if graph:
-            graph.note_mat(self)
+        vals = self._device_values()
+        with _MAT_LOCK:
+            vals.memset(0)
+            graph = _state.get('capturing')
+            self._zeroed = graph if graph else True
+            if graph:
+                graph.note_mat(self)
 
     def _known_zero(self):
         return self._zeroed is (_state.get('capturing') or True)
@@ -714,10 +723,11 @@ class Mat(DeviceDataMixin, base.Mat):
             raise IndexError("zero_rows: row %d outside [0, %d)" % (bad, nrows))
         rows = rows.astype(np.int32)
         vals = self._device_values()
-        self._written()
-        call("op2b_mat_zero_rows", vals.ptr, self._sparsity._d_rowptr, self._sparsity._d_colidx,
-             nrows, rows.ctypes.data_as(C.POINTER(C.c_int32)), rows.size, float(diag_val),
-             self.dtype.itemsize, 0)
+        with _MAT_LOCK:
+            self._written()
+            call("op2b_mat_zero_rows", vals.ptr, self._sparsity._d_rowptr, self._sparsity._d_colidx,
+                 nrows, rows.ctypes.data_as(C.POINTER(C.c_int32)), rows.size, float(diag_val),
+                 self.dtype.itemsize, 0)
 
     def _assemble(self):
         pass
@@ -2110,12 +2120,30 @@ class _BoundLoop(object):
             if ptr != self._gptr[k]:
                 struct.pack_into("<Q", buf, off, ptr)
                 self._gptr[k] = ptr
-        mod = self.module
         if self.consts:
-            _sync_consts(mod, self.consts)
+            _sync_consts(self.module, self.consts)
+        if self.mats:
+            with _MAT_LOCK:
+                launched = self._issue(buf, rng)
+        else:
+            launched = self._issue(buf, rng)
+        if not launched:
+            return
+        for d in self._written:
+            d._state = DEVICE
+            d._wgen += 1
+            if d._data.flags.writeable:      # unlike setflags, cheap to ask
+                maybe_setflags(d._data, write=False)
+        for k in self._reducing:
+            args[self._gbl[k][1]].data._state = DEVICE
+
+    def _issue(self, buf, rng):
+        """Launch what the parameter block ``buf`` describes (False: there are no
+        elements); the Mats are not known to be zero any more."""
+        zero = {id(m): m._known_zero() for m in self.mats}
         if self.row_blocks is not None:
             for j, m in enumerate(self.mats):
-                z = 1 if m._known_zero() else 0
+                z = int(zero[id(m)])
                 if z != self._mzero[j]:
                     struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), z)
                     self._mzero[j] = z
@@ -2126,47 +2154,40 @@ class _BoundLoop(object):
                 raise DeviceError("element range %s of a %s-form loop" % (rng, self.spec.mode))
             n = rng[1] - rng[0]
         if n == 0:
-            return
-        params = buf
+            return False
+        for m in self.mats:
+            m._state = DEVICE
+            m._written()
+        fn = self.module.fn
         if self.indirect:
             plan = self.plan
-            call("op2b_launch_colored", mod.fn, plan.ncolors, plan.ncolblk_host, self.block_size,
-                 self.smem, 0, params, self.layout.nbytes, codegen.ParamLayout.COL_OFFSET)
+            call("op2b_launch_colored", fn, plan.ncolors, plan.ncolblk_host, self.block_size,
+                 self.smem, 0, buf, self.layout.nbytes, codegen.ParamLayout.COL_OFFSET)
         elif rng is not None:
             # the header's (start, end) for this launch only: the launch
             # copies the parameter block when it is issued
             struct.pack_into("<qq", buf, 16, rng[0], rng[1])
             try:
-                call("op2b_launch", mod.fn, self.grid, self.block_size, self.launch_smem, 0,
-                     params, self.layout.nbytes)
+                call("op2b_launch", fn, self.grid, self.block_size, self.launch_smem, 0,
+                     buf, self.layout.nbytes)
             finally:
                 struct.pack_into("<qq", buf, 16, 0, self.range_end)
         else:
             call("op2b_launch_record", self._desc_ptr)
         if self.spec.mode == "lma":
             kahan = 1 if self.kahan else 0            # OP2B_LMA_KAHAN
-            for buf, inc, target, cdim, ntargets, arity, mask in self.lma:
+            for contrib, inc, target, cdim, ntargets, arity, mask in self.lma:
                 if isinstance(target, Mat):
                     out = target._device_values().ptr
                     # Mat incidences hold contribution indices (OP2B_LMA_MAT_INDEX);
                     # a Mat known to be zero needs no read of its values
                     # (OP2B_LMA_FROM_ZERO)
-                    flags = kahan | 4 | (2 if target._known_zero() else 0)
-                    target._written()
+                    flags = kahan | 4 | (2 if zero[id(target)] else 0)
                 else:
                     out, flags = target._device.ptr, kahan
-                call("op2b_lma_reduce", out, cdim, inc.ptr, inc.list, ntargets, buf.ptr, n,
+                call("op2b_lma_reduce", out, cdim, inc.ptr, inc.list, ntargets, contrib.ptr, n,
                      arity, mask, flags, 0)
-        for d in self._written:
-            d._state = DEVICE
-            d._wgen += 1
-            if d._data.flags.writeable:      # unlike setflags, cheap to ask
-                maybe_setflags(d._data, write=False)
-        for k in self._reducing:
-            args[self._gbl[k][1]].data._state = DEVICE
-        for m in self.mats:
-            m._state = DEVICE
-            m._written()
+        return True
 
 
 _ENV = {"gen": None, "key": None}
@@ -2595,11 +2616,15 @@ class Graph(object):
         self._mats[id(m)] = weakref.ref(m)
 
     def launch(self):
-        call("op2b_graph_launch", self.handle, 0)
-        for ref in self._mats.values():
-            m = ref()
-            if m is not None:
-                m._written()
+        if not self._mats:
+            call("op2b_graph_launch", self.handle, 0)
+            return
+        with _MAT_LOCK:
+            for ref in self._mats.values():
+                m = ref()
+                if m is not None:
+                    m._written()
+            call("op2b_graph_launch", self.handle, 0)
 
     def close(self):
         """Destroy the executable graph now rather than at collection."""

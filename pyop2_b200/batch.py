@@ -424,6 +424,18 @@ class BatchLoop(object):
             for inst in self.instances:
                 inst.sync()
         b200._sync_consts(self.module, self.consts)
+        if self._mats:
+            with b200._MAT_LOCK:
+                for m in self._mats:
+                    m._written()
+                self._issue()
+        else:
+            self._issue()
+        if sync_host:
+            for inst in self.instances:
+                inst.mark()
+
+    def _issue(self):
         if self.form == "color":
             for grid, params in self._colour_launches:
                 call("op2b_launch", self.module.fn, grid, self.spec.block_size, self.smem, 0,
@@ -433,11 +445,6 @@ class BatchLoop(object):
                  self._params, self.layout.nbytes)
         if self.has_fin and self.nsegs:
             call("op2b_launch", self.fin, self.fin_grid, 256, 0, 0, self._params, self.layout.nbytes)
-        for m in self._mats:
-            m._written()
-        if sync_host:
-            for inst in self.instances:
-                inst.mark()
 
 
 _PLANS = {}

@@ -100,3 +100,33 @@ def test_a_loop_changes_form_while_threads_run_it(backend, monkeypatch):
         forms = [b.spec.mode for b in b200.ParLoop._bound_cache.values() if b.mats == [mat]]
         assert forms == ["rowblk"]
         np.testing.assert_array_equal(mat.array, 41 * one.array)
+
+
+@pytest.mark.parametrize("runs", [0, 1 << 30])
+def test_threads_add_to_a_mat_just_zeroed(backend, monkeypatch, runs):
+    """Loops of several threads into one zeroed Mat (row blocks; or two of them row
+    blocks and two the element form): the first write ends what is known of it,
+    whoever makes it, so nothing is added to a zero that has gone."""
+    from pyop2_b200 import b200, op2
+    from pyop2_b200.workloads import meshes
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
+    coords, elem = meshes.rect_p1(30, 21, 2)
+    el, nd = op2.Set(len(elem), 1, "el"), op2.Set(len(coords), 1, "nd")
+    m = op2.Map(el, nd, 3, elem, "m")
+    w = op2.Dat(el, np.arange(1.0, 1 + len(elem)), np.float64, "w")
+    ks = [op2.Kernel("void adds%d(double A[1][1], double *w, int i, int j) { A[0][0] += %d * w[0]; }" % (k, 10 ** k),
+                     "adds%d" % k) for k in range(4)]
+    mat = op2.Mat(op2.Sparsity((m, m), "s"), np.float64, "mat")
+
+    def assemble(k):
+        op2.par_loop(ks[k], el(3, 3), mat((m[op2.i[0]], m[op2.i[1]]), op2.INC), w(op2.IdentityMap, op2.READ))
+        return True
+    for k in range(4):
+        monkeypatch.setattr(b200, "_ROWBLK_RUNS", 0 if k < 2 else runs)
+        assemble(k)
+    monkeypatch.setattr(b200, "_ROWBLK_RUNS", 1 << 30)
+    want = mat.array
+    for _ in range(50):
+        mat.zero()
+        assert in_threads(4, assemble) == [True] * 4
+        np.testing.assert_array_equal(mat.array, want)
