@@ -2692,10 +2692,12 @@ def _relaxed_exec(graph, trace, small_only=False):
 
 def _rows_before_capture():
     """Build the row blocks of the assembly loops that ran just before: a
-    graph is recorded to be replayed, and cannot change its loops' form."""
-    since = _runs[0] - _ROWBLK_RECENT
+    graph is recorded to be replayed, and cannot change its loops' form.  Loops
+    bound under another configuration or other Consts are left alone: the graph
+    would not use them, and they would be bound with the options of now."""
+    since, env = _runs[0] - _ROWBLK_RECENT, _env_key()
     for bl in list(ParLoop._bound_cache.values()):
-        if bl._rows_later and bl._last_run > since:
+        if bl._rows_later and bl._last_run > since and bl.key[-1] == env:
             new = bl._in_rows(bl._args)
             # now, not as copies in the graph: the new form's module has not run
             _sync_consts(new.module, new.consts)

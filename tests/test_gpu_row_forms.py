@@ -1,0 +1,56 @@
+"""When an assembly loop takes the row block form, and which one."""
+
+import numpy as np
+import pytest
+
+from pyop2_b200 import configuration as cfg
+from pyop2_b200.workloads import fem, meshes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def op2(backend, monkeypatch):
+    """Row blocks at any size, before a capture only."""
+    from pyop2_b200 import b200, op2
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
+    monkeypatch.setattr(b200, "_ROWBLK_RUNS", 1 << 30)
+    return op2
+
+
+def problem(op2, nx=11, ny=9):
+    coords, elem = meshes.rect_p1(nx, ny, 1)
+    return fem.build_p1(op2, 0, coords=coords, elem=elem, stiffness=True)
+
+
+def bound(name, iterset):
+    from pyop2_b200 import b200
+    return [b for b in b200.ParLoop._bound_cache.values()
+            if b.spec.kernel_name == name and b.iterset is iterset]
+
+
+@pytest.mark.parametrize("other", [{"inc_mode": "color"}, {"inc_mode": "lma", "kahan": True}, {"fmad": True}])
+def test_a_capture_leaves_loops_of_another_configuration(op2, other):
+    """What ran under other options is not bound again with those of the capture."""
+    from pyop2_b200 import b200
+    P = problem(op2)
+    cfg.configure(inc_mode="staged", kahan=False, fmad=False)
+    fem.assemble_p1(op2, P)
+    (mass,) = bound("p1_mass", P.elements)
+    assert mass.spec.mode == "atomic"
+    cfg.configure(**other)
+    P.b.zero()
+    with b200.capture() as g:
+        P.b.zero()
+    assert bound("p1_mass", P.elements) == [mass] and mass.spec.mode == "atomic" and mass.row_blocks is None
+    cfg.configure(inc_mode="staged", kahan=False, fmad=False)
+    with b200.capture() as g:
+        P.mat.zero()
+        fem.assemble_p1(op2, P)
+    (rows,) = bound("p1_mass", P.elements)
+    assert rows.spec.mode == "rowblk" and not rows.spec.rowblk["kahan"] and not rows.spec.fmad
+    g.launch()
+    want = P.mat.array
+    P.mat.zero()
+    fem.assemble_p1(op2, P)
+    np.testing.assert_array_equal(P.mat.array, want)
