@@ -116,6 +116,8 @@ _SIGS = {
 
 EXPORTED = tuple(sorted(_SIGS))
 
+ERR_NOMEM = 4     # OP2B_ERR_NOMEM
+
 _lib = None
 
 
@@ -144,14 +146,14 @@ def last_error():
 
 def check(rc, what=""):
     if rc != 0:
-        raise DeviceError("%s: %s" % (what, last_error()))
+        raise DeviceError("%s: %s" % (what, last_error()), rc)
 
 
 def call(name, *args):
     """Call entry point ``name`` and raise DeviceError on a non-zero status."""
     rc = getattr(_lib, name)(*args)
     if rc != 0:
-        raise DeviceError("%s failed (status %d): %s" % (name, rc, last_error()))
+        raise DeviceError("%s failed (status %d): %s" % (name, rc, last_error()), rc)
     return rc
 
 

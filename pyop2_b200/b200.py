@@ -1773,7 +1773,9 @@ class _BoundLoop(object):
             try:
                 form = row_block_spec(spec, specs, maps, mats,
                                       kahan=spec.mode == "lma" and cfg.cfg['kahan'])
-            except DeviceError as e:          # no memory for the tables
+            except DeviceError as e:
+                if e.status != _lib.ERR_NOMEM:      # else: no memory for the tables
+                    raise
                 debug("row blocks of %s: %s" % (loop.kernel.name, e))
                 form = None
             if form is not None:

@@ -48,6 +48,8 @@ int set_error(int code, const char *fmt, ...) {
 int check_cuda(cudaError_t err, const char *what) {
   if (err == cudaSuccess) return OP2B_OK;
   int code = (err == cudaErrorMemoryAllocation) ? OP2B_ERR_NOMEM : OP2B_ERR_CUDA;
+  // a caller may go on without the memory: its next launch is not to be told of it
+  if (code == OP2B_ERR_NOMEM) cudaGetLastError();
   return set_error(code, "%s failed: %s (%s)", what, cudaGetErrorString(err),
                    cudaGetErrorName(err));
 }
@@ -118,7 +120,10 @@ struct Slab {
       if (cudaStreamIsCapturing(g_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
         return nullptr;
       void *p = nullptr;
-      if (cudaMallocAsync(&p, (size_t)kSlabBlocks * kSlabBytes, g_stream) != cudaSuccess) return nullptr;
+      if (cudaMallocAsync(&p, (size_t)kSlabBlocks * kSlabBytes, g_stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+      }
       base = static_cast<char *>(p);
       device = g_device;
       for (nfree = 0; nfree < kSlabBlocks; ++nfree) free_list[nfree] = (uint16_t)(kSlabBlocks - 1 - nfree);
@@ -422,7 +427,13 @@ int op2b_memcpy_d2h(void *dst, uint64_t src, uint64_t bytes, uint64_t stream) {
   if (!bytes) return OP2B_OK;
   cudaStream_t s = stream_of(stream);
   void *to = dst;
-  if (bytes <= 256 && (t_small.p || cudaMallocHost(&t_small.p, 256) == cudaSuccess)) to = t_small.p;
+  if (bytes <= 256) {
+    if (!t_small.p && cudaMallocHost(&t_small.p, 256) != cudaSuccess) {
+      t_small.p = nullptr;
+      cudaGetLastError();
+    }
+    if (t_small.p) to = t_small.p;
+  }
   OP2B_CUDA(cudaMemcpyAsync(to, reinterpret_cast<const void *>(src), bytes,
                             cudaMemcpyDeviceToHost, s));
   OP2B_CUDA(cudaStreamSynchronize(s));

@@ -62,4 +62,9 @@ class MapValueError(ValueError):
 
 
 class DeviceError(RuntimeError):
-    """A call into the B200 device library failed (CUDA, NVRTC, bad handle)."""
+    """A call into the B200 device library failed (CUDA, NVRTC, bad handle).
+    ``status``: the library's status, 0 where the error was found before a call."""
+
+    def __init__(self, message="", status=0):
+        RuntimeError.__init__(self, message)
+        self.status = status

@@ -54,3 +54,49 @@ def test_a_capture_leaves_loops_of_another_configuration(op2, other):
     P.mat.zero()
     fem.assemble_p1(op2, P)
     np.testing.assert_array_equal(P.mat.array, want)
+
+
+
+def test_what_ends_a_build(op2, monkeypatch):
+    """Without memory for the tables a loop keeps the element form; any other
+    failure of the build is reported."""
+    from pyop2_b200 import b200
+    from pyop2_b200.exceptions import DeviceError
+
+    def fail(status):
+        def of(*args):
+            e = DeviceError("op2b_row_blocks_build failed")
+            e.status = status
+            raise e
+        monkeypatch.setattr(b200.RowBlocks, "of", of)
+    P = problem(op2, 8, 5)
+    fem.assemble_p1(op2, P)
+    want = P.mat.array
+    fail(1)
+    with pytest.raises(DeviceError):
+        with b200.capture():
+            pass
+    P = problem(op2, 8, 5)
+    fail(4)
+    fem.assemble_p1(op2, P)
+    with b200.capture() as g:
+        P.mat.zero()
+        fem.assemble_p1(op2, P)
+    assert [b.spec.mode for b in bound("p1_mass", P.elements)] == ["atomic"]
+    g.launch()
+    np.testing.assert_allclose(P.mat.array, want, rtol=1e-14)
+
+
+def test_an_allocation_that_failed_is_over(backend):
+    """Its error is the failing call's own: what runs next is not told of it."""
+    from pyop2_b200 import b200
+    from pyop2_b200._lib import call
+    from pyop2_b200.exceptions import DeviceError
+    x = b200._upload(np.arange(50.0))
+    with pytest.raises(DeviceError) as e:
+        b200.DeviceBuffer(1 << 50)
+    assert e.value.status == 4
+    call("op2b_vec_binop", x.ptr, x.ptr, 0, 2.0, 50, 2, 0, 0)     # checks its launch's error
+    got = np.zeros(50)
+    x.to_host(got)
+    np.testing.assert_array_equal(got, 2 * np.arange(50.0))
