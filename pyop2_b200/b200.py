@@ -648,7 +648,13 @@ _MAT_LOCK = threading.RLock()
 
 
 class Mat(DeviceDataMixin, base.Mat):
-    """Device CSR values on a Sparsity."""
+    """Device CSR values on a Sparsity.
+
+    An assembly that owns the values does not read those of a Mat known to be
+    zero: a fresh one, or one not written since :meth:`zero` by a loop, a graph,
+    a batch, :meth:`zero_rows` or through :meth:`_device_values`.  Whoever writes
+    through an address kept from before the last :meth:`zero` (a tensor view, a
+    batch instance patched to it) has to take it again after the write."""
 
     def __init__(self, sparsity, dtype=None, name=None):
         base.Mat.__init__(self, sparsity, dtype, name)
@@ -660,12 +666,20 @@ class Mat(DeviceDataMixin, base.Mat):
         # what the same graph does next, not for anything run now
         self._zeroed = True
 
-    def _device_values(self):
+    def _values(self):
         if self._vals is None:
             self._vals = DeviceBuffer(max(self._sparsity.nz, 1) * self.dtype.itemsize)
             self._vals.memset(0)
             self._state = DEVICE
         return self._vals
+
+    def _device_values(self):
+        """The values' device memory, to read or write: they are not known to be
+        zero after that."""
+        vals = self._values()
+        with _MAT_LOCK:
+            self._written()
+        return vals
 
     @property
     def array(self):
@@ -689,7 +703,7 @@ class Mat(DeviceDataMixin, base.Mat):
         return ret
 
     def zero(self):
-        vals = self._device_values()
+        vals = self._values()
         with _MAT_LOCK:
             vals.memset(0)
             graph = _state.get('capturing')
@@ -722,7 +736,7 @@ class Mat(DeviceDataMixin, base.Mat):
             bad = rows[(rows < 0) | (rows >= nrows)][0]
             raise IndexError("zero_rows: row %d outside [0, %d)" % (bad, nrows))
         rows = rows.astype(np.int32)
-        vals = self._device_values()
+        vals = self._values()
         with _MAT_LOCK:
             self._written()
             call("op2b_mat_zero_rows", vals.ptr, self._sparsity._d_rowptr, self._sparsity._d_colidx,
@@ -764,7 +778,7 @@ class Solver(base.Solver):
         b._to_device()
         if x._state is DEVICE_UNALLOCATED:
             x._allocate_device()
-        vals = A._device_values()
+        vals = A._values()
         max_it = int(p['maximum_iterations'])
         hist = np.zeros(max_it + 1, dtype=np.float64)
         its, reason = C.c_int32(), C.c_int32()
@@ -1861,7 +1875,7 @@ class _BoundLoop(object):
         for k, m in enumerate(maps):
             vals["m%d" % k] = m._to_device().ptr
         for j, m in enumerate(mats):
-            vals["mv%d" % j] = m._device_values().ptr
+            vals["mv%d" % j] = m._values().ptr
             vals["mr%d" % j] = m.sparsity._d_rowptr
             vals["mc%d" % j] = m.sparsity._d_colidx
         if spec.mat_slots:
@@ -2180,7 +2194,7 @@ class _BoundLoop(object):
             kahan = 1 if self.kahan else 0            # OP2B_LMA_KAHAN
             for contrib, inc, target, cdim, ntargets, arity, mask in self.lma:
                 if isinstance(target, Mat):
-                    out = target._device_values().ptr
+                    out = target._values().ptr
                     # Mat incidences hold contribution indices (OP2B_LMA_MAT_INDEX);
                     # a Mat known to be zero needs no read of its values
                     # (OP2B_LMA_FROM_ZERO)

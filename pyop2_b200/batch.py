@@ -91,7 +91,7 @@ def _bind(fields):
             vals[name] = o._to_device().ptr
         elif kind == "mat":
             j = name[2:]
-            vals[name] = o._device_values().ptr
+            vals[name] = o._values().ptr
             vals["mr" + j] = o.sparsity._d_rowptr
             vals["mc" + j] = o.sparsity._d_colidx
         elif kind == "slots":

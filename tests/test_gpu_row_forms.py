@@ -100,3 +100,37 @@ def test_an_allocation_that_failed_is_over(backend):
     got = np.zeros(50)
     x.to_host(got)
     np.testing.assert_array_equal(got, 2 * np.arange(50.0))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_values_written_at_their_address(op2, monkeypatch, graph):
+    """Values written through an address taken after the zeroing, or taken again
+    after the write, are added to."""
+    from pyop2_b200 import b200
+    from pyop2_b200._lib import call
+    monkeypatch.setattr(b200, "_ROWBLK_RUNS", 0)
+    P = problem(op2, 10, 6)
+    loop = lambda: fem.assemble_p1_stiffness(op2, P)  # noqa: E731
+    loop()
+    assert [b.spec.mode for b in bound("p1_stiff", P.elements)] == ["rowblk"]
+    one = P.stiff.array
+    fives = np.full_like(one, 5.0)
+
+    def write(ptr):
+        call("op2b_memcpy_h2d", ptr, fives.ctypes.data, fives.nbytes, 0)
+    if graph:
+        with b200.capture() as g:
+            loop()
+        run = g.launch
+    else:
+        run = loop
+    P.stiff.zero()
+    write(P.stiff._device_values().ptr)
+    run()
+    np.testing.assert_allclose(P.stiff.array, one + fives, rtol=1e-14)
+    kept = P.stiff._device_values().ptr
+    P.stiff.zero()
+    write(kept)
+    P.stiff._device_values()
+    run()
+    np.testing.assert_allclose(P.stiff.array, one + fives, rtol=1e-14)
