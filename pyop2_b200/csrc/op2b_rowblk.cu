@@ -50,6 +50,7 @@
 #include <cstring>
 
 #include "op2b_internal.h"
+#include "op2b_rowblk_room.h"
 #include "op2b_scan.cuh"
 
 namespace op2b {
@@ -84,8 +85,9 @@ struct RbArgs {
   int32_t *scal;               // see kS*
 };
 
-// device scalars
-enum { kSFlag, kSCursor, kSMaxPacket, kSMaxTargets, kSScan = kSMaxTargets + kRbStages, kSBlocks = kSScan + 3,
+// device scalars; the cursor has 64 bits, since what the blocks take may be past
+// what a directory entry can hold
+enum { kSCursor, kSFlag = kSCursor + 2, kSMaxPacket, kSMaxTargets, kSScan = kSMaxTargets + kRbStages, kSBlocks = kSScan + 3,
        kSUsed, kSMaxItems, kSMaxRows, kSChanged, kSCount = kSChanged + 3 };
 
 constexpr int kRbLevels = 32;          // levels told apart in a region's order
@@ -430,20 +432,22 @@ __global__ void __launch_bounds__(kRbThreads) rb_build_kernel(const RbArgs A) {
   __syncthreads();
   nlids = s_ids;
   const int nshort = ne - nlong - nempty;
-  __shared__ int s_start;
-  const int u_elems = A.ids ? rb_units(4 * NE) : 0, u_items = rb_units(2 * ra * NE), u_shorts = rb_units(8LL * nshort), u_longs = rb_units(8LL * nlong);
+  __shared__ int64_t s_start;
+  const int u_elems = A.ids ? rb_units(4 * NE) : 0, u_items = rb_units(2 * ra * NE);
+  const int u_shorts = rb_units(8LL * nshort), u_longs = rb_units(8LL * nlong);
   int head = 2 + u_elems + u_items + u_longs + rb_units(2LL * nlids);
   for (int s = 0; s < A.st.n; ++s) head += rb_units(4 * nt[s]) + rb_units(2 * A.st.arity[s] * NE);
   const int total = head + u_shorts;
   if (tid == 0) {
-    s_start = atomicAdd(&A.scal[kSCursor], total);
-    A.dir[blk] = make_int2(s_start, (int)((unsigned)head | (unsigned)total << 16));
+    s_start = (int64_t)atomicAdd(reinterpret_cast<unsigned long long *>(A.scal + kSCursor),
+                                 (unsigned long long)total);
+    A.dir[blk] = make_int2((int)s_start, (int)((unsigned)head | (unsigned)total << 16));
     atomicMax(&A.scal[kSMaxPacket], head);
     for (int s = 0; s < A.st.n; ++s) atomicMax(&A.scal[kSMaxTargets + s], nt[s]);
     if ((int64_t)ns * ca > 65535 || total > 65535) atomicExch(&A.scal[kSFlag], 1);
   }
   __syncthreads();
-  if ((int64_t)s_start + total > A.cap) return;    // the host allocates what the cursor says and repeats
+  if (s_start + total > A.cap) return;    // the host allocates what the cursor says and repeats
   uint4 *P = A.pkt + s_start;
   if (tid == 0) {
     P[0] = make_uint4(NE, nshort, nlong, ni);
@@ -642,12 +646,7 @@ int op2b_row_blocks_build(uint64_t rmap_, uint64_t cmap_, int32_t nelem, int32_t
   A.scal = scal;
   RB_TRY(dev_alloc((void **)&P->dir, sizeof(int2) * (size_t)nblocks, s));
   A.dir = P->dir;
-  // room for elements shared by 1.7 blocks and targets by 2; what the blocks
-  // really take is known after the first pass
-  const int64_t nent = h[kSScan + 1];
-  int64_t staged = 0;
-  for (int q = 0; q < nstage; ++q) staged += 4 * 2 * (int64_t)nrows + 2 * stage_arity[q] * nelem * 17 / 10;
-  A.cap = ((4 * A.ids + 2 * ra) * (int64_t)nelem * 17 / 10 + staged + 8 * nent + tot * ca / 2) / 16 + (int64_t)nblocks * (7 + 2 * nstage);
+  A.cap = row_block_room(nelem, ra, ca, nrows, h[kSScan + 1], nblocks, A.ids, nstage, stage_arity);
   RB_CUDA(cudaFuncSetAttribute(rb_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int attempt = 0; attempt < 2; ++attempt) {
     if (A.cap >= INT_MAX) return done(OP2B_OK, false);
@@ -658,11 +657,13 @@ int op2b_row_blocks_build(uint64_t rmap_, uint64_t cmap_, int32_t nelem, int32_t
     RB_CUDA(cudaMemcpyAsync(h, scal, sizeof h, cudaMemcpyDeviceToHost, s));
     RB_CUDA(cudaStreamSynchronize(s));
     if (h[kSFlag]) return done(OP2B_OK, false);
-    if (h[kSCursor] <= A.cap) break;
-    A.cap = h[kSCursor];
+    int64_t taken;
+    memcpy(&taken, h + kSCursor, sizeof taken);
+    if (taken <= A.cap) break;
+    A.cap = taken;
     dev_free(P->pkt, s);
     P->pkt = nullptr;
-    RB_CUDA(cudaMemsetAsync(scal + kSCursor, 0, sizeof(int32_t), s));
+    RB_CUDA(cudaMemsetAsync(scal + kSCursor, 0, sizeof(int64_t), s));
   }
   P->nblocks = nblocks;
   P->max_items = A.max_items;
