@@ -110,15 +110,17 @@ struct Slab {
   int device = -1, nfree = 0;
   uint16_t free_list[kSlabBlocks];
 
+  // The library's stream is being recorded into a graph, whose allocations belong
+  // to the graph and whose work may run again whenever it is launched.
+  static bool capturing() {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(g_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+  }
   // Null: the caller allocates.
   void *take(uint64_t bytes) {
-    if (bytes > kSlabBytes) return nullptr;
+    if (bytes > kSlabBytes || capturing()) return nullptr;
     std::lock_guard<std::mutex> lock(m);
     if (!base) {
-      // never inside a graph recording, whose allocations belong to the graph
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(g_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
-        return nullptr;
       void *p = nullptr;
       if (cudaMallocAsync(&p, (size_t)kSlabBlocks * kSlabBytes, g_stream) != cudaSuccess) {
         cudaGetLastError();
@@ -131,11 +133,13 @@ struct Slab {
     if (device != g_device || nfree == 0) return nullptr;
     return base + (size_t)free_list[--nfree] * kSlabBytes;
   }
+  // False: p is not of the slab.  A block released while a graph is recorded is
+  // not handed out again: the graph may go on writing it.
   bool give(void *p) {
     std::lock_guard<std::mutex> lock(m);
     const char *c = static_cast<char *>(p);
     if (!base || c < base || c >= base + (size_t)kSlabBlocks * kSlabBytes) return false;
-    free_list[nfree++] = (uint16_t)((c - base) / kSlabBytes);
+    if (!capturing()) free_list[nfree++] = (uint16_t)((c - base) / kSlabBytes);
     return true;
   }
   void shutdown() {

@@ -49,3 +49,29 @@ def test_fresh_globals_of_a_repeated_reduction(op2):
         else:
             assert g.data[0] == n + 499500.0
     assert [g.data[0] for _, g in kept] == [n + 499500.0 for n, _ in kept]
+
+
+def test_blocks_released_in_a_capture(op2):
+    """What a recorded loop writes is not handed to another Global, even if its own
+    Global is dropped before the recording ends."""
+    from pyop2_b200 import b200
+    s = op2.Set(500, 1, "s")
+    d = op2.Dat(s, np.arange(500.0), np.float64, "d")
+    k = op2.Kernel("void addup(double *x, double *g) { *g += *x; }", "addup")
+    g = op2.Global(1, 0.0, np.float64, "g")
+    add = lambda v: op2.par_loop(k, s, d(op2.IdentityMap, op2.READ), v(op2.INC))  # noqa: E731
+    add(g)
+    ptr = g._device.ptr
+    with b200.capture() as graph:
+        add(g)
+        del g
+    more = [b200.DeviceBuffer(8) for _ in range(300)]
+    assert ptr not in {b.ptr for b in more}
+    zero = np.zeros(1)
+    for b in more:
+        b.from_host(zero)
+    graph.launch()
+    graph.launch()
+    for b in more:
+        b.to_host(zero)
+        assert zero[0] == 0.0
