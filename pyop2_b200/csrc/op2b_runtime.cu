@@ -109,6 +109,7 @@ struct Slab {
   char *base = nullptr;
   int device = -1, nfree = 0;
   uint16_t free_list[kSlabBlocks];
+  bool held[kSlabBlocks] = {};
 
   // The library's stream is being recorded into a graph, whose allocations belong
   // to the graph and whose work may run again whenever it is launched.
@@ -131,16 +132,22 @@ struct Slab {
       for (nfree = 0; nfree < kSlabBlocks; ++nfree) free_list[nfree] = (uint16_t)(kSlabBlocks - 1 - nfree);
     }
     if (device != g_device || nfree == 0) return nullptr;
-    return base + (size_t)free_list[--nfree] * kSlabBytes;
+    const int k = free_list[--nfree];
+    held[k] = true;
+    return base + (size_t)k * kSlabBytes;
   }
-  // False: p is not of the slab.  A block released while a graph is recorded is
-  // not handed out again: the graph may go on writing it.
-  bool give(void *p) {
+  // 0: p is not of the slab; 1: given back; -1: p is not a block that is held.  A
+  // block released while a graph is recorded is not handed out again: the graph
+  // may go on writing it.
+  int give(void *p) {
     std::lock_guard<std::mutex> lock(m);
     const char *c = static_cast<char *>(p);
-    if (!base || c < base || c >= base + (size_t)kSlabBlocks * kSlabBytes) return false;
-    if (!capturing()) free_list[nfree++] = (uint16_t)((c - base) / kSlabBytes);
-    return true;
+    if (!base || c < base || c >= base + (size_t)kSlabBlocks * kSlabBytes) return 0;
+    const size_t k = (c - base) / kSlabBytes;
+    if (!held[k] || (c - base) % kSlabBytes) return -1;
+    held[k] = false;
+    if (!capturing()) free_list[nfree++] = (uint16_t)k;
+    return 1;
   }
   void shutdown() {
     std::lock_guard<std::mutex> lock(m);
@@ -400,7 +407,9 @@ int op2b_malloc(uint64_t *dptr, uint64_t bytes) {
 int op2b_free(uint64_t dptr) {
   OP2B_REQUIRE_INIT();
   void *p = reinterpret_cast<void *>(dptr);
-  if (p && !g_slab.give(p)) OP2B_CUDA(cudaFreeAsync(p, g_stream));
+  const int given = p ? g_slab.give(p) : 1;
+  if (given < 0) return set_error(OP2B_ERR_ARG, "op2b_free: %p is not an allocated block", p);
+  if (given == 0) OP2B_CUDA(cudaFreeAsync(p, g_stream));
   return OP2B_OK;
 }
 

@@ -75,3 +75,24 @@ def test_blocks_released_in_a_capture(op2):
     for b in more:
         b.to_host(zero)
         assert zero[0] == 0.0
+
+
+def test_what_is_not_a_held_block_is_refused(op2):
+    """A small block given back twice, or an address inside one: refused, and the
+    slab stays as it was."""
+    from pyop2_b200._lib import call
+    from pyop2_b200.b200 import DeviceBuffer
+    from pyop2_b200.exceptions import DeviceError
+    keep = DeviceBuffer(64)
+    b = DeviceBuffer(64)
+    with pytest.raises(DeviceError):
+        call("op2b_free", b.ptr + 16)
+    call("op2b_free", b.ptr)
+    for _ in range(3):
+        with pytest.raises(DeviceError):
+            call("op2b_free", b.ptr)
+    b.ptr = 0
+    ptrs = [keep.ptr]
+    more = [DeviceBuffer(64) for _ in range(300)]
+    ptrs += [m.ptr for m in more]
+    assert len(set(ptrs)) == 301
