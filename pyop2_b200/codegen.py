@@ -698,6 +698,7 @@ def _atomic_body(spec):
     coloured form (OP2 leaves their conflicts to the user)."""
     bs = spec.block_size
     L = ["extern \"C\" __global__ void %s %s(const op2b_params p) {" % (_bounds(spec), stub_name(spec))]
+    _gbl_prologue(spec, L)
     if spec.itspace_split:
         # warp w evaluates block (w mod Q) of the local positions of the 32
         # elements 32 * (w div Q) + lane (the block is warp-uniform)
@@ -720,7 +721,6 @@ def _atomic_body(spec):
         L.append("  }")
         L.append("}")
         return "\n".join(L)
-    _gbl_prologue(spec, L)
     L.append("  for (op2b_i64 e = p.start + (op2b_i64)blockIdx.x * %d + threadIdx.x; e < p.end;"
              " e += (op2b_i64)gridDim.x * %d) {" % (bs, bs))
     L += _atomic_element(spec, "    ")
