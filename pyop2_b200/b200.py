@@ -1190,6 +1190,12 @@ def _incidence(m):
 class RowBlocks(object):
     """Row blocks of a scalar Mat assembly (op2b_row_blocks_build)."""
 
+    def forget(self, sparsity):
+        """Not kept with the Sparsity any more (loops that use them hold them)."""
+        tables = sparsity.__dict__["_row_block_tables"]
+        for key in [k for k, hit in tables.items() if hit[0] is self]:
+            del tables[key]
+
     @classmethod
     def of(cls, sparsity, rmap, cmap, region, stage_maps, ids):
         """The row blocks of assembly through (rmap, cmap), with the elements'
@@ -1236,14 +1242,39 @@ _ROWBLK_THREADS = 128
 _ROWBLK_BYTES = 18 << 10
 
 
-# contributions a launch adds, below which the form makes too little difference
-# for its tables (0.4 ms to build).  In a graph with the memsets and P1's RHS,
-# element form against row blocks: P1 256 x 256 (1.2 million) 14.3 us against 13.0
-# with structured numbering and 17.8 against 14.6 permuted, 222 x 222 (0.9 million)
-# 12.4 against 12.4 and 14.5 against 14.5; P2 128 x 128 (1.2 million) 20.6 against
-# 16.5, 91 x 91 (0.6 million) 14.5 against 12.4, 64 x 64 (0.3 million) 11.1
-# against 9.8
+# contributions a launch adds from which the form is tried.  Below, it changes a
+# launch by less than 3 us either way (zeroed, P1 222 x 222, 0.9 million: 12.3 us and
+# 12.3; P2 91 x 91 K + M, 0.6 million: 16.4 and 14.3; added to values they hold: 10.2
+# and 12.3; 14.3 and 12.3) and its tables take 0.7 ms and more to build
 _ROWBLK_MIN = 1 << 20
+
+# From so many contributions on both forms are timed (see _BoundLoop._faster_form):
+# sizes and types do not say which is faster.  Row blocks evaluate an element once
+# for every block that owns one of its rows (1.27 times on P1 triangles, 1.67 on P2,
+# 2.5 on P1 tetrahedra, 3.1 on Q1 hexahedra, 4.4 on P2 tetrahedra), which is hidden
+# behind memory traffic or not, by the kernel's cost; and they read values that the
+# element form's reductions only add to.  Element form against row blocks, us, of
+# zeroed Mats (with their memsets) and of Mats that hold values:
+#   P1 mass 256 x 256           12.3    12.3       12.3    14.3
+#   P1 mass 512 x 512           28.6    24.6       26.6    30.7
+#   P1 mass 1000 x 1000        108.5    69.6      100.4   112.6
+#   P2 K + M 181 x 181          38.9    26.6       32.8    26.5
+#   P2 K + M 1024 x 1024      1050     518        936     672
+#   P1 tetrahedra 64^3, mass   143     129        139     139
+#     the same, stiffness      145     193        139     205
+#   Q1 hexahedra 64^3, mass    133      90        125      96
+#     the same, stiffness at 8 points
+#                             6503   16935       6483   16927
+_TRIAL_MIN = 1 << 20
+_TRIAL_RUNS = 6
+# Of the element form's time that row blocks may take, zeroed and holding values.
+# The runs timed find in L2 what others may have driven out, and row blocks read
+# more (P1 724 x 724 holding values: 46.3 and 47.6 us, after a flush 61 and 70)
+_TRIAL_ZEROED, _TRIAL_HOLDING = 0.97, 0.9
+# Two-phase sums: 18.9 million contributions take op2b_lma_reduce 119 us, whatever
+# the kernel, where the contributions do not fit the L2.  Row blocks that take no
+# longer are not compared with them.
+_LMA_PER_MS = 159e6
 
 # runs of a bound loop before its row blocks are built: the build takes what 30
 # (P2) to 80 (P1) runs then save, and the element form needs only the slot table,
@@ -1757,10 +1788,11 @@ class _BoundLoop(object):
     """Everything about a par_loop that does not change between calls with
     the same objects: generated stub, plan, parameter block."""
 
-    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None, rows=False, sums=True):
+    def __init__(self, loop, inc_mode=None, owner_mode=None, nelem=None, rows=None, sums=True):
         # nelem: bind to the set's first nelem elements only (the core of a
-        # partitioned set, run in the staged form); rows: in the row block form
-        # if it runs the loop; sums: the summing staged form may be taken
+        # partitioned set, run in the staged form); rows: True in the row block
+        # form if it runs the loop, False never; sums: the summing staged form may
+        # be taken
         info = loop_spec(loop, inc_mode=inc_mode, owner_mode=owner_mode, size=nelem, sums=sums)
         spec = info['spec']
         specs = info['specs']
@@ -1769,16 +1801,18 @@ class _BoundLoop(object):
         iterset = info['iterset']
         args = loop.args
         self.row_blocks = None
+        self._element = None    # what runs instead while a Mat holds values
         self.room = 0       # 16-byte units of a packet (row blocks, summing staged form)
         self._runs, self._last_run = 0, -_ROWBLK_RECENT
         self.key = None     # in ParLoop._bound_cache
+        self._buf = None    # parameter block (see _prepare)
         self._written = []
         # Mat assembly by the owners of the rows (see codegen._rowblk_body): at
         # once in place of the two-phase form, whose own tables cost as much to
         # build; else when the loop has run often enough (see run)
         w = next((s for s in specs if s.kind == "mat"), None)
         self._rows_later = bool(
-            w is not None and nelem is None and inc_mode is None and not _partitioned(iterset)
+            w is not None and rows is not False and nelem is None and inc_mode is None and not _partitioned(iterset)
             and (spec.mode == "lma" or (spec.mode == "atomic" and _default_mat_form()))
             and iterset.size * w.arity * w.carity >= _ROWBLK_MIN
             and codegen.rowblk_capable(spec))
@@ -2086,12 +2120,70 @@ class _BoundLoop(object):
         if new.row_blocks is None:
             return self
         new.key = self.key
-        new._prepare(loop)
+        new = self._faster_form(new, loop)
         if ParLoop._bound_cache.get(self.key) is self:
             ParLoop._bound_cache[self.key] = new
         return new
 
+    def _faster_form(self, rows, loop):
+        """``rows`` (this loop in the row block form) or this bound loop, whichever
+        takes less time; ``rows`` may run this one while the Mats hold values.
+        Timed into stand-ins for the Mats, the only data such a loop writes."""
+        for bl in (self, rows):
+            if bl._buf is None:
+                bl._prepare(loop)
+        if sum(m.sparsity.nz for m in self.mats) == 0 or self._contributions() < _TRIAL_MIN:
+            return rows
+        try:
+            stand_ins = [DeviceBuffer(m._values().nbytes) for m in self.mats]
+        except DeviceError as e:
+            if e.status != _lib.ERR_NOMEM:
+                raise
+            stand_ins = None
+        if stand_ins:
+            ms = self._device_ms(loop.args, stand_ins)
+            if rows._device_ms(loop.args, stand_ins, zero=True) < _TRIAL_ZEROED * ms:
+                if rows._device_ms(loop.args, stand_ins) >= _TRIAL_HOLDING * ms:
+                    rows._element = self
+                return rows
+        rows.row_blocks.forget(self.mats[0].sparsity)
+        return self
+
+    def _contributions(self):
+        w = next(a for a in self.spec.args if a.kind == "mat")
+        return self.nelem * w.arity * w.carity
+
+    def _device_ms(self, args, stand_ins, zero=False):
+        """Device time of a run that writes ``stand_ins`` for the Mats."""
+        if self.consts:
+            _sync_consts(self.module, self.consts)
+        buf = C.create_string_buffer(self._buf.raw, self.layout.nbytes)
+        for off, ai, _ in self._gbl:
+            g = args[ai].data
+            g._to_device()
+            struct.pack_into("<Q", buf, off, g._device.ptr)
+        for j, b in enumerate(stand_ins):
+            struct.pack_into("<Q", buf, self.layout.offset("mv%d" % j), b.ptr)
+            if self.row_blocks is not None:
+                struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), int(zero))
+
+        def run():
+            call("op2b_launch", self.module.fn, self.grid, self.block_size, self.launch_smem, 0, buf,
+                 self.layout.nbytes)
+            if self.spec.mode == "lma":
+                self._reduce([b.ptr for b in stand_ins], [zero] * len(stand_ins))
+        run()
+        e0 = Event().record()
+        for _ in range(_TRIAL_RUNS):
+            run()
+        e1 = Event().record()
+        e1.synchronize()
+        return e0.elapsed_ms(e1) / _TRIAL_RUNS
+
     def _run(self, loop, rng=None):
+        if self._element is not None and not all(m._known_zero() for m in self.mats):
+            self._element._run(loop, rng)
+            return
         _runs[0] += 1
         if self._rows_later:
             self._runs += 1
@@ -2101,7 +2193,7 @@ class _BoundLoop(object):
                 if form is not self:
                     form._run(loop)
                     return
-        if getattr(self, "_buf", None) is None:
+        if self._buf is None:
             self._prepare(loop)
         for d in self.dats:
             st = d._state
@@ -2191,19 +2283,23 @@ class _BoundLoop(object):
         else:
             call("op2b_launch_record", self._desc_ptr)
         if self.spec.mode == "lma":
-            kahan = 1 if self.kahan else 0            # OP2B_LMA_KAHAN
-            for contrib, inc, target, cdim, ntargets, arity, mask in self.lma:
-                if isinstance(target, Mat):
-                    out = target._values().ptr
-                    # Mat incidences hold contribution indices (OP2B_LMA_MAT_INDEX);
-                    # a Mat known to be zero needs no read of its values
-                    # (OP2B_LMA_FROM_ZERO)
-                    flags = kahan | 4 | (2 if zero[id(target)] else 0)
-                else:
-                    out, flags = target._device.ptr, kahan
-                call("op2b_lma_reduce", out, cdim, inc.ptr, inc.list, ntargets, contrib.ptr, n,
-                     arity, mask, flags, 0)
+            self._reduce([m._values().ptr for m in self.mats], [zero[id(m)] for m in self.mats])
         return True
+
+    def _reduce(self, values, zero):
+        """The second phase of the two-phase form, into the Mats' ``values``
+        (``zero``: known to be zero) and the Dats."""
+        kahan = 1 if self.kahan else 0            # OP2B_LMA_KAHAN
+        for k, (contrib, inc, target, cdim, ntargets, arity, mask) in enumerate(self.lma):
+            if isinstance(target, Mat):           # in the order of self.mats, before the Dats
+                # Mat incidences hold contribution indices (OP2B_LMA_MAT_INDEX);
+                # a Mat known to be zero needs no read of its values
+                # (OP2B_LMA_FROM_ZERO)
+                out, flags = values[k], kahan | 4 | (2 if zero[k] else 0)
+            else:
+                out, flags = target._device.ptr, kahan
+            call("op2b_lma_reduce", out, cdim, inc.ptr, inc.list, ntargets, contrib.ptr, self.nelem,
+                 arity, mask, flags, 0)
 
 
 _ENV = {"gen": None, "key": None}
@@ -2491,7 +2587,31 @@ def _bind(loop, iterset):
             if cb is not None and cb.spec.mode == "staged":
                 bl.core_loop = cb
         return bl
-    return _bind_fitting(loop) or _BoundLoop(loop, inc_mode='atomic')
+    bl = _bind_fitting(loop) or _BoundLoop(loop, inc_mode='atomic')
+    if bl.row_blocks is not None and not _state.get('capturing'):
+        return _row_blocks_or_two_phases(bl, loop)
+    return bl
+
+
+def _row_blocks_or_two_phases(rows, loop):
+    """A loop bound at once as row blocks (inc_mode='lma'), or in the two-phase form
+    where that is faster: both add in the same order.  Where its contributions
+    would not fit the L2, only kernels that cost more than the second phase's sums
+    are worth its tables."""
+    rows._prepare(loop)
+    added = rows._contributions() * len(rows.mats)
+    if rows._contributions() < _TRIAL_MIN:
+        return rows
+    try:
+        if 8 * added > _state['l2_bytes'] // 2:
+            ms = rows._device_ms(loop.args, [DeviceBuffer(m._values().nbytes) for m in rows.mats])
+            if ms <= added / _LMA_PER_MS:
+                return rows
+        return _BoundLoop(loop, rows=False)._faster_form(rows, loop)
+    except DeviceError as e:
+        if e.status != _lib.ERR_NOMEM:
+            raise
+        return rows
 
 
 class ParLoop(base.ParLoop):

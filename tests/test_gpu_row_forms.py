@@ -134,3 +134,59 @@ def test_values_written_at_their_address(op2, monkeypatch, graph):
     P.stiff._device_values()
     run()
     np.testing.assert_allclose(P.stiff.array, one + fives, rtol=1e-14)
+
+
+def hexes(n):
+    """(points, elem) of n^3 cubes."""
+    i, j, k = np.meshgrid(*[np.arange(n)] * 3, indexing="ij")
+    at = lambda a, b, c: ((i + a) * (n + 1) + j + b) * (n + 1) + k + c  # noqa: E731
+    elem = np.stack([at(a, b, c) for a in (0, 1) for b in (0, 1) for c in (0, 1)], -1).reshape(-1, 8)
+    return (n + 1) ** 3, elem.astype(np.int32)
+
+
+# per entry: whole numbers, exact in any order; the second after a chain of 400
+# dependent divisions, and so dearer than anything else in the launch
+CHEAP = "A[0][0] += w[0] * (1 + 3 * i + j);"
+DEAR = "double s = 1 + w[0] + i * j; for (int q = 0; q < 400; ++q) s = 3.0 / s; " + CHEAP[:-1] + " + (s == 0.0);"
+
+
+@pytest.mark.parametrize("inc_mode,other", [("staged", "atomic"), ("lma", "lma")])
+@pytest.mark.parametrize("cost,code,zeroed", [("cheap", CHEAP, True), ("dear", DEAR, False)])
+def test_the_faster_form_runs(backend, monkeypatch, inc_mode, other, cost, code, zeroed):
+    """Row blocks evaluate an element of a hexahedral mesh about three times: loops
+    whose kernel outweighs the rest keep the form that evaluates it once.  The
+    results are those of a loop that never had the choice."""
+    from pyop2_b200 import b200, op2
+    nodes, elem = hexes(27)
+    n = len(elem)
+    assert n * 64 >= b200._TRIAL_MIN
+    cfg.configure(inc_mode=inc_mode, kahan=False)
+    el, nd = op2.Set(n, 1, "el"), op2.Set(nodes, 1, "nd")
+    m = op2.Map(el, nd, 8, elem, "m")
+    w = op2.Dat(el, np.random.default_rng(3).integers(1, 9, n).astype(np.float64), np.float64, "w")
+    g = op2.Global(1, 2.0, np.float64, "g")
+    sp = op2.Sparsity((m, m), "s")
+    mats = [op2.Mat(sp, np.float64, "m%d" % k) for k in range(2)]
+    k = op2.Kernel("void %s(double A[1][1], double *w, double *g, int i, int j) { %s A[0][0] += g[0]; }"
+                   % (cost, code), cost)
+
+    def assemble(mat):
+        op2.par_loop(k, el(8, 8), mat((m[op2.i[0]], m[op2.i[1]]), op2.INC), w(op2.IdentityMap, op2.READ),
+                     g(op2.READ))
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 1 << 40)
+    assemble(mats[0])
+    assemble(mats[0])
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 1 << 20)
+    mat = mats[1]
+    assemble(mat)
+    with b200.capture() as graph:
+        mat.zero()
+        assemble(mat)
+    assemble(mat)
+    np.testing.assert_array_equal(mat.array, mats[0].array)
+    graph.launch()
+    assemble(mat)
+    np.testing.assert_array_equal(mat.array, mats[0].array)
+    (bl,) = [b for b in bound(cost, el) if b.mats[0] is mat]
+    assert bl.spec.mode == ("rowblk" if zeroed else other)
+    assert bl._element is None or bl._element.spec.mode == other
