@@ -645,6 +645,7 @@ class Sparsity(base.Sparsity):
 # changes with it: another thread's loop, issued between the two, would take a Mat
 # for zero that no longer is (or the other way round)
 _MAT_LOCK = threading.RLock()
+_PREPARE_LOCK = threading.RLock()     # held while a bound loop is prepared
 
 
 class Mat(DeviceDataMixin, base.Mat):
@@ -2035,6 +2036,14 @@ class _BoundLoop(object):
                 return False
         return True
 
+    def _ready(self, loop):
+        """Prepared, once: the launch record points into the parameter block, so
+        no second one may take its place while another thread launches."""
+        if self._buf is None:
+            with _PREPARE_LOCK:
+                if self._buf is None:
+                    self._prepare(loop)
+
     def _prepare(self, loop):
         """First run: device copies of the Dats, the full parameter block in a
         persistent buffer, and the bookkeeping later runs need."""
@@ -2082,16 +2091,16 @@ class _BoundLoop(object):
         self._mzero = [0] * len(self.mats)
         self._written = [d for d in self.dats if any(m != "READ" for m in self.dat_access[id(d)])]
         self._reducing = [k for k, (_, _, red) in enumerate(self._gbl) if red]
-        n = self.nelem
-        self._buf = C.create_string_buffer(self.layout.pack(n, 0, self.range_end, vals),
-                                           self.layout.nbytes)
+        buf = C.create_string_buffer(self.layout.pack(self.nelem, 0, self.range_end, vals),
+                                     self.layout.nbytes)
         if self.room:
             # the header's second colour field: room of a packet
-            struct.pack_into("<i", self._buf, codegen.ParamLayout.COL_OFFSET + 4, self.room)
+            struct.pack_into("<i", buf, codegen.ParamLayout.COL_OFFSET + 4, self.room)
         # op2b_launch_desc of the launches over the whole set
-        self._desc = C.create_string_buffer(struct.pack("<QQIIII", self.module.fn, C.addressof(self._buf),
+        self._desc = C.create_string_buffer(struct.pack("<QQIIII", self.module.fn, C.addressof(buf),
                                                         self.grid, self.block_size, self.launch_smem, 0))
         self._desc_ptr = C.addressof(self._desc)
+        self._buf = buf       # last: other threads run the loop from here on
 
     def run(self, loop, rng=None):
         """Run the loop over its whole set, or over elements [start, end)
@@ -2130,8 +2139,7 @@ class _BoundLoop(object):
         takes less time; ``rows`` may run this one while the Mats hold values.
         Timed into stand-ins for the Mats, the only data such a loop writes."""
         for bl in (self, rows):
-            if bl._buf is None:
-                bl._prepare(loop)
+            bl._ready(loop)
         if sum(m.sparsity.nz for m in self.mats) == 0 or self._contributions() < _TRIAL_MIN:
             return rows
         try:
@@ -2193,8 +2201,7 @@ class _BoundLoop(object):
                 if form is not self:
                     form._run(loop)
                     return
-        if self._buf is None:
-            self._prepare(loop)
+        self._ready(loop)
         for d in self.dats:
             st = d._state
             if st is HOST:
@@ -2598,7 +2605,7 @@ def _row_blocks_or_two_phases(rows, loop):
     where that is faster: both add in the same order.  Where its contributions
     would not fit the L2, only kernels that cost more than the second phase's sums
     are worth its tables."""
-    rows._prepare(loop)
+    rows._ready(loop)
     added = rows._contributions() * len(rows.mats)
     if rows._contributions() < _TRIAL_MIN:
         return rows

@@ -130,3 +130,25 @@ def test_threads_add_to_a_mat_just_zeroed(backend, monkeypatch, runs):
         mat.zero()
         assert in_threads(4, assemble) == [True] * 4
         np.testing.assert_array_equal(mat.array, want)
+
+
+def test_threads_run_a_loop_for_the_first_time(backend):
+    """One of them prepares it; the others launch what it prepared."""
+    from pyop2_b200 import b200, op2
+    n = 3000
+    s = op2.Set(n, 1, "s")
+    k = op2.Kernel("void first(double *x, double *g) { *x += 1; }", "first")
+    g = op2.Global(1, 1.0, np.float64, "g")
+    for _ in range(40):
+        d = op2.Dat(s, np.zeros(n), np.float64, "d")
+        b200.ParLoop._bound_cache.clear()
+        loop = b200.ParLoop(k, s, d(op2.IdentityMap, op2.RW), g(op2.READ))
+        d._to_device(), g._to_device()
+        bl = loop._bound()
+
+        def work(_):
+            for _ in range(5):
+                bl.run(loop)
+            return True
+        assert in_threads(4, work) == [True] * 4
+        np.testing.assert_array_equal(d.data.ravel(), np.full(n, 20.0))
