@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <unistd.h>
 #include <nvrtc.h>
+#include <pthread.h>
 
 #include <algorithm>
 #include <atomic>
@@ -216,9 +217,15 @@ struct CopyPool {
     }
   }
 };
-// Never destroyed: a process may end with the threads asleep in it.
+// Never destroyed: a process may end with the threads asleep in it.  A fork takes
+// the mutex first, so that the child, which copies alone, does not find it held by
+// a thread it does not have.
 static CopyPool &copy_pool() {
-  static CopyPool *p = new CopyPool;
+  static CopyPool *p = [] {
+    pthread_atfork([] { copy_pool().m.lock(); }, [] { copy_pool().m.unlock(); },
+                   [] { copy_pool().m.unlock(); });
+    return new CopyPool;
+  }();
   return *p;
 }
 
