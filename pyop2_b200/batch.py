@@ -309,7 +309,7 @@ class BatchLoop(object):
         self.config = dict(block_size=spec.block_size, elems_per_thread=spec.batch,
                            min_blocks=spec.min_blocks, ctas_per_sm=int(ctas_per_sm))
         if self.form == "color":
-            self.config = dict(form="color", part_size=spec.batch_part_size,
+            self.config = dict(form="color", part_size=self.instances[0].spec.batch_part_size,
                                block_size=spec.block_size, min_blocks=spec.min_blocks,
                                ctas_per_sm=int(ctas_per_sm))
         self.smem = max((i.plan.nshared for i in self.instances if i.plan is not None), default=0)
