@@ -68,12 +68,12 @@ int op2b_memcpy_d2h(void *dst, uint64_t src, uint64_t bytes, uint64_t stream);
  * stream as a pageable-memory copy does.  No reference counterpart (PyCUDA
  * copied Globals with synchronous memcpy_htod, pyop2/cuda.py:325-340). */
 int op2b_memcpy_h2d_small(uint64_t dst, const void *src, uint64_t bytes, uint64_t stream);
-/* Device-to-host copy that returns at once (stream-ordered; complete when an
- * event recorded after it completes).  dst must be pinned host memory
- * (op2b_host_alloc) for the copy to be asynchronous. */
 /* Host copies of n arrays (dst[i], src[i]: host addresses, no overlap), shared from
  * 1 MB on between the caller and up to seven threads kept for it. */
 int op2b_host_copy(int32_t n, const uint64_t *dst, const uint64_t *src, const uint64_t *bytes);
+/* Device-to-host copy that returns at once (stream-ordered; complete when an
+ * event recorded after it completes).  dst must be pinned host memory
+ * (op2b_host_alloc) for the copy to be asynchronous. */
 int op2b_memcpy_d2h_async(void *dst, uint64_t src, uint64_t bytes, uint64_t stream);
 int op2b_memcpy_d2d(uint64_t dst, uint64_t src, uint64_t bytes, uint64_t stream);
 int op2b_memset(uint64_t dst, int value, uint64_t bytes, uint64_t stream);

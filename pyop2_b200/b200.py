@@ -913,8 +913,9 @@ class RegionPlan(object):
         sinc = (C.c_int32 * max(ns, 1))(*[1 if (stage_inc is None or f) else 0
                                           for f in (stage_inc or [1] * ns)])
         h = C.c_uint64()
-        call("op2b_region_plan_build_even" if even else "op2b_region_plan_build", set_size, part_size, region_size, grow_map._to_device().ptr,
-             grow_map.dim, grow_map.dataset.total_size, ns, smap, sar, sinc, 0, C.byref(h))
+        call("op2b_region_plan_build_even" if even else "op2b_region_plan_build", set_size, part_size,
+             region_size, grow_map._to_device().ptr, grow_map.dim, grow_map.dataset.total_size, ns, smap,
+             sar, sinc, 0, C.byref(h))
         self._handle = h.value
         if bank_slots:
             call("op2b_region_plan_bank_slots", self._handle, 0)

@@ -25,7 +25,6 @@ synchronise per colour).  Per element the stub:
   the device (op2b_device.cuh: op2b_reduce).
 """
 
-import copy
 import os
 import re
 import struct

@@ -87,8 +87,19 @@ struct RbArgs {
 
 // device scalars; the cursor has 64 bits, since what the blocks take may be past
 // what a directory entry can hold
-enum { kSCursor, kSFlag = kSCursor + 2, kSMaxPacket, kSMaxTargets, kSScan = kSMaxTargets + kRbStages, kSBlocks = kSScan + 3,
-       kSUsed, kSMaxItems, kSMaxRows, kSChanged, kSCount = kSChanged + 3 };
+enum {
+  kSCursor,
+  kSFlag = kSCursor + 2,
+  kSMaxPacket,
+  kSMaxTargets,
+  kSScan = kSMaxTargets + kRbStages,
+  kSBlocks = kSScan + 3,
+  kSUsed,
+  kSMaxItems,
+  kSMaxRows,
+  kSChanged,
+  kSCount = kSChanged + 3
+};
 
 constexpr int kRbLevels = 32;          // levels told apart in a region's order
 
