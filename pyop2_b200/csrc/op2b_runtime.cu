@@ -49,8 +49,9 @@ int set_error(int code, const char *fmt, ...) {
 int check_cuda(cudaError_t err, const char *what) {
   if (err == cudaSuccess) return OP2B_OK;
   int code = (err == cudaErrorMemoryAllocation) ? OP2B_ERR_NOMEM : OP2B_ERR_CUDA;
-  // a caller may go on without the memory: its next launch is not to be told of it
-  if (code == OP2B_ERR_NOMEM) cudaGetLastError();
+  // the caller is told here and may go on (without the memory, or from a finaliser):
+  // the next launch is not to be told again
+  cudaGetLastError();
   return set_error(code, "%s failed: %s (%s)", what, cudaGetErrorString(err),
                    cudaGetErrorName(err));
 }

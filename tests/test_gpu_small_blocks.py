@@ -96,3 +96,20 @@ def test_what_is_not_a_held_block_is_refused(op2):
     more = [DeviceBuffer(64) for _ in range(300)]
     ptrs += [m.ptr for m in more]
     assert len(set(ptrs)) == 301
+
+
+def test_large_blocks_released_in_a_capture(op2):
+    """Memory of the allocator cannot be released while its stream is recorded; the
+    refusal is that call's own, and the recording and later launches go on."""
+    from pyop2_b200 import b200
+    from pyop2_b200._lib import call
+    n = 400
+    x, big = b200._upload(np.arange(float(n))), b200.DeviceBuffer(1 << 16)
+    with b200.capture() as graph:
+        del big
+        call("op2b_vec_binop", x.ptr, x.ptr, 0, 2.0, n, 2, 0, 0)     # checks its launch's error
+    graph.launch()
+    call("op2b_vec_binop", x.ptr, x.ptr, 0, 1.0, n, 0, 0, 0)
+    got = np.zeros(n)
+    x.to_host(got)
+    np.testing.assert_array_equal(got, 2 * np.arange(float(n)) + 1)
