@@ -484,7 +484,7 @@ def run_gpu(args, ws, rank, local):
                            "alone_ms": round(ms, 4)}
     # the form res_calc ran in (before other legs bind loops of that kernel)
     res_form = _RES_FORM.get(_loop_mode("res_calc"), "all colour launches")
-    # one-off cost of the staged form: building res_calc's locality partition
+    # one-off cost of the staged form: building res_calc's locality partition and packets
     partition_ms = None
     staged = [bl for bl in b200.ParLoop._bound_cache.values()
               if bl.spec.kernel_name == "res_calc" and bl.spec.mode == "staged"]
@@ -492,8 +492,11 @@ def run_gpu(args, ws, rank, local):
         rp = staged[-1].region_plan
         b200.synchronize()
         t0 = time.perf_counter()
-        b200.RegionPlan(rp.set_size, rp.part_size, rp.region_size, rp._keep[0], rp._keep[1:],
-                        rp.stage_inc, even=rp.even)
+        plan = b200.RegionPlan(rp.set_size, rp.part_size, rp.region_size, rp._keep[0], rp._keep[1:],
+                               rp.stage_inc, even=rp.even)
+        region = staged[-1].spec.region
+        if region.get("sums"):          # and the packets the summing form walks
+            plan.packets(region["inc_stages"], region["ids"])
         b200.synchronize()
         partition_ms = round((time.perf_counter() - t0) * 1e3, 3)
     res_bytes = bytes_["res_calc"]
