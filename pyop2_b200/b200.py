@@ -2123,8 +2123,12 @@ class _BoundLoop(object):
     def _in_rows(self, args):
         """The loop bound in the row block form, which takes this bound loop's
         place in the cache; this one where that form does not run the loop.  It
-        stays as it is, since another thread may be running it."""
-        self._rows_later, self._args = False, None
+        stays as it is, since another thread may be running it, and one thread does
+        this once."""
+        with _PREPARE_LOCK:
+            if not self._rows_later:
+                return self
+            self._rows_later, self._args = False, None
         loop = _Loop(self._again[0], self._again[1], args)
         new = _BoundLoop(loop, rows=True)
         if new.row_blocks is None:

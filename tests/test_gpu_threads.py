@@ -102,6 +102,42 @@ def test_a_loop_changes_form_while_threads_run_it(backend, monkeypatch):
         np.testing.assert_array_equal(mat.array, 41 * one.array)
 
 
+def test_one_thread_binds_the_row_blocks(backend, monkeypatch):
+    """Threads that find at once that a loop has run often enough: one of them builds
+    and times, the others go on in the element form."""
+    from pyop2_b200 import b200, op2
+    from pyop2_b200.workloads import meshes
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
+    monkeypatch.setattr(b200, "_ROWBLK_RUNS", 1)
+    coords, elem = meshes.rect_p1(40, 31, 2)
+    el, nd = op2.Set(len(elem), 1, "el"), op2.Set(len(coords), 1, "nd")
+    m = op2.Map(el, nd, 3, elem, "m")
+    w = op2.Dat(el, np.ones(len(elem)), np.float64, "w")
+    mat = op2.Mat(op2.Sparsity((m, m), "s"), np.float64, "mat")
+    k = op2.Kernel("void once(double A[1][1], double *w, int i, int j) { A[0][0] += w[0] * (1 + i + j); }", "once")
+
+    def assemble(_):
+        op2.par_loop(k, el(3, 3), mat((m[op2.i[0]], m[op2.i[1]]), op2.INC), w(op2.IdentityMap, op2.READ))
+        return True
+    assemble(0)
+    want = mat.array
+    here, timed = threading.Barrier(4), []
+    bind, choose = b200._BoundLoop._in_rows, b200._BoundLoop._faster_form
+
+    def together(self, args):
+        here.wait(30)
+        return bind(self, args)
+
+    def counted(self, rows, loop):
+        timed.append(rows)
+        return choose(self, rows, loop)
+    monkeypatch.setattr(b200._BoundLoop, "_in_rows", together)
+    monkeypatch.setattr(b200._BoundLoop, "_faster_form", counted)
+    assert in_threads(4, assemble) == [True] * 4
+    assert len(timed) == 1
+    np.testing.assert_array_equal(mat.array, 5 * want)
+
+
 @pytest.mark.parametrize("runs", [0, 1 << 30])
 def test_threads_add_to_a_mat_just_zeroed(backend, monkeypatch, runs):
     """Loops of several threads into one zeroed Mat (row blocks; or two of them row
