@@ -1268,7 +1268,9 @@ _ROWBLK_MIN = 1 << 20
 #     the same, stiffness at 8 points
 #                             6503   16935       6483   16927
 _TRIAL_MIN = 1 << 20
-_TRIAL_RUNS = 6
+# the mean of so many runs; a run of more than _TRIAL_LONG ms is long enough to be
+# told from another by itself (the Q1 stiffness above: 47 ms for both forms, not 164)
+_TRIAL_RUNS, _TRIAL_LONG = 6, 2.0
 # Of the element form's time that row blocks may take, zeroed and holding values.
 # The runs timed find in L2 what others may have driven out, and row blocks read
 # more (P1 724 x 724 holding values: 46.3 and 47.6 us, after a flush 61 and 70)
@@ -2185,13 +2187,18 @@ class _BoundLoop(object):
                  self.layout.nbytes)
             if self.spec.mode == "lma":
                 self._reduce([b.ptr for b in stand_ins], [zero] * len(stand_ins))
-        run()
-        e0 = Event().record()
-        for _ in range(_TRIAL_RUNS):
+
+        def timed(runs):
+            e0 = Event().record()
+            for _ in range(runs):
+                run()
+            e1 = Event().record()
+            e1.synchronize()
+            return e0.elapsed_ms(e1) / runs
+        with _MAT_LOCK:      # other threads' assembly would be timed with it
             run()
-        e1 = Event().record()
-        e1.synchronize()
-        return e0.elapsed_ms(e1) / _TRIAL_RUNS
+            first = timed(1)
+            return first if first > _TRIAL_LONG else timed(_TRIAL_RUNS)
 
     def _run(self, loop, rng=None):
         if self._element is not None and not all(m._known_zero() for m in self.mats):

@@ -190,3 +190,23 @@ def test_the_faster_form_runs(backend, monkeypatch, inc_mode, other, cost, code,
     (bl,) = [b for b in bound(cost, el) if b.mats[0] is mat]
     assert bl.spec.mode == ("rowblk" if zeroed else other)
     assert bl._element is None or bl._element.spec.mode == other
+
+
+@pytest.mark.parametrize("long,runs", [(1e9, 2 + 6), (0.0, 2)])
+def test_long_runs_are_timed_once(op2, monkeypatch, long, runs):
+    """Two forms, zeroed and (where row blocks win that) holding values."""
+    from pyop2_b200 import b200
+    monkeypatch.setattr(b200, "_TRIAL_MIN", 0)
+    monkeypatch.setattr(b200, "_TRIAL_LONG", long)
+    P = problem(op2)
+    fem.assemble_p1(op2, P)
+    want = P.mat.array
+    made, call = [], b200.call
+    monkeypatch.setattr(b200, "call", lambda name, *a: (made.append(name), call(name, *a))[1])
+    with b200.capture() as g:
+        P.mat.zero()
+    n = made.count("op2b_launch")
+    assert n in (2 * runs, 3 * runs)
+    P.mat.zero()
+    fem.assemble_p1(op2, P)
+    np.testing.assert_allclose(P.mat.array, want, rtol=1e-14)
