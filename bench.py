@@ -643,12 +643,13 @@ _RES_FORM = {"staged": "one launch over the locality partition", "atomic": "one 
 
 def _loop_mode(kernel_name):
     """The form (staged / atomic / plan ...) the backend chose for the most
-    recently bound loop of a kernel."""
+    recently bound loop of a kernel; of a Mat assembly, the one that runs while
+    its Mats hold values, as the timed loops find them."""
     from pyop2_b200 import b200
     mode = None
     for bl in b200.ParLoop._bound_cache.values():
         if bl.spec.kernel_name == kernel_name:
-            mode = bl.spec.mode
+            mode = (bl._element or bl).spec.mode
     return mode
 
 
