@@ -23,14 +23,15 @@ keys of the B200 backend:
   every contribution, then each target adds its contributions in element
   order -- the sequential backend's order -- optionally Kahan-compensated;
   deterministic and independent of the launch configuration; large scalar Mat
-  assembly adds them in the same order by row blocks, without the store;
+  assembly adds them in the same order by row blocks, without the store, where
+  that is faster;
   loops it cannot run fall back to ``'color'``) or ``'staged'`` (one launch over a locality
   partition: the set is reordered into compact regions grown on the GPU,
   each block's distinct targets are staged in shared memory and INC rows
   summed there, then added once per target with atomics; summation
   order varies between runs within rounding; loops without indirect INC,
-  with Mats, or whose staged rows would not fit a CTA's shared memory run
-  as ``'atomic'``) or ``'gather'`` (loops whose only writes are INC into
+  with Mats, or whose staged rows would not fit a CTA's shared memory (nor
+  without the room that summing takes beside them) run as ``'atomic'``) or ``'gather'`` (loops whose only writes are INC into
   one Dat through one Map: one thread per target walks the target's
   incidence in element order, evaluates the kernel for each incident element
   and keeps its own share, then writes the target once -- no atomics, no
@@ -73,8 +74,8 @@ keys of the B200 backend:
 * ``mat_slots``: (with this, ``mat_per_entry``, ``mat_slots_rel`` and
   ``itspace_split`` at their defaults, large scalar Mat assembly that keeps
   running, or is about to be recorded in a graph, is run by the owners of the
-  rows instead: every stored entry written once, its contributions added in
-  element order) assemble scalar Mats in the atomic form through a cached
+  rows where that is faster: every stored entry written once, its contributions
+  added in element order; both ways are timed once) assemble scalar Mats in the atomic form through a cached
   scatter-slot table (the CSR position of every element's local entries,
   built once per Sparsity and Map pair: nelem x arity^2 int32 of device
   memory) instead of searching the CSR row for every entry;
