@@ -2168,8 +2168,9 @@ class _BoundLoop(object):
         w = next(a for a in self.spec.args if a.kind == "mat")
         return self.nelem * w.arity * w.carity
 
-    def _device_ms(self, args, stand_ins, zero=False):
-        """Device time of a run that writes ``stand_ins`` for the Mats."""
+    def _device_ms(self, args, stand_ins, zero=False, enough=0.0):
+        """Device time of a run that writes ``stand_ins`` for the Mats; that of the
+        first one, which is no shorter, if it is at most ``enough`` ms."""
         if self.consts:
             _sync_consts(self.module, self.consts)
         buf = C.create_string_buffer(self._buf.raw, self.layout.nbytes)
@@ -2196,7 +2197,9 @@ class _BoundLoop(object):
             e1.synchronize()
             return e0.elapsed_ms(e1) / runs
         with _MAT_LOCK:      # other threads' assembly would be timed with it
-            run()
+            first = timed(1)
+            if first <= enough:
+                return first
             first = timed(1)
             return first if first > _TRIAL_LONG else timed(_TRIAL_RUNS)
 
@@ -2623,9 +2626,11 @@ def _row_blocks_or_two_phases(rows, loop):
         return rows
     try:
         if 8 * added > _state['l2_bytes'] // 2:
-            ms = rows._device_ms(loop.args, [DeviceBuffer(m._values().nbytes) for m in rows.mats])
-            if ms <= added / _LMA_PER_MS:
+            most = added / _LMA_PER_MS
+            stand_ins = [DeviceBuffer(m._values().nbytes) for m in rows.mats]
+            if rows._device_ms(loop.args, stand_ins, enough=most) <= most:
                 return rows
+            del stand_ins
         return _BoundLoop(loop, rows=False)._faster_form(rows, loop)
     except DeviceError as e:
         if e.status != _lib.ERR_NOMEM:

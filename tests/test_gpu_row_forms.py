@@ -210,3 +210,18 @@ def test_long_runs_are_timed_once(op2, monkeypatch, long, runs):
     P.mat.zero()
     fem.assemble_p1(op2, P)
     np.testing.assert_allclose(P.mat.array, want, rtol=1e-14)
+
+
+def test_row_blocks_within_the_second_phase_run_once(op2, monkeypatch):
+    """What the first run shows is not measured again."""
+    from pyop2_b200 import b200
+    monkeypatch.setattr(b200, "_TRIAL_MIN", 0)
+    monkeypatch.setattr(b200, "_LMA_PER_MS", 1e-6)
+    monkeypatch.setitem(b200._state, "l2_bytes", 0)
+    cfg.configure(inc_mode="lma")
+    P = problem(op2)
+    made, call = [], b200.call
+    monkeypatch.setattr(b200, "call", lambda name, *a: (made.append(name), call(name, *a))[1])
+    fem.assemble_p1_stiffness(op2, P)
+    assert [b.spec.mode for b in bound("p1_stiff", P.elements)] == ["rowblk"]
+    assert made.count("op2b_launch") == 1
