@@ -704,9 +704,9 @@ class Mat(DeviceDataMixin, base.Mat):
         return ret
 
     def zero(self):
-        vals = self._values()
+        vals = self._vals or self._values()
         with _MAT_LOCK:
-            vals.memset(0)
+            call("op2b_memset", vals.ptr, 0, vals.nbytes, 0)
             graph = _state.get('capturing')
             self._zeroed = graph if graph else True
             if graph:
@@ -2092,6 +2092,9 @@ class _BoundLoop(object):
                 self._ginit.append(None)
         self._gflag = [0] * len(self._gbl)
         self._mzero = [0] * len(self.mats)
+        # what is known of the Mats changes the launch; the record is all there is
+        self._uses_zero = self.row_blocks is not None or self.spec.mode == "lma"
+        self._one_record = not self.indirect and self.spec.mode != "lma" and self.nelem > 0
         self._written = [d for d in self.dats if any(m != "READ" for m in self.dat_access[id(d)])]
         self._reducing = [k for k, (_, _, red) in enumerate(self._gbl) if red]
         buf = C.create_string_buffer(self.layout.pack(self.nelem, 0, self.range_end, vals),
@@ -2216,7 +2219,8 @@ class _BoundLoop(object):
                 if form is not self:
                     form._run(loop)
                     return
-        self._ready(loop)
+        if self._buf is None:
+            self._ready(loop)
         for d in self.dats:
             st = d._state
             if st is HOST:
@@ -2255,9 +2259,11 @@ class _BoundLoop(object):
         if self.mats:
             with _MAT_LOCK:
                 launched = self._issue(buf, rng)
-        else:
-            launched = self._issue(buf, rng)
-        if not launched:
+            if not launched:
+                return
+        elif self._one_record and rng is None:      # the common case, without a call
+            call("op2b_launch_record", self._desc_ptr)
+        elif not self._issue(buf, rng):
             return
         for d in self._written:
             d._state = DEVICE
@@ -2270,10 +2276,11 @@ class _BoundLoop(object):
     def _issue(self, buf, rng):
         """Launch what the parameter block ``buf`` describes (False: there are no
         elements); the Mats are not known to be zero any more."""
-        zero = {id(m): m._known_zero() for m in self.mats}
+        if self._uses_zero:
+            zero = [m._known_zero() for m in self.mats]
         if self.row_blocks is not None:
-            for j, m in enumerate(self.mats):
-                z = int(zero[id(m)])
+            for j, z in enumerate(zero):
+                z = int(z)
                 if z != self._mzero[j]:
                     struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), z)
                     self._mzero[j] = z
@@ -2285,9 +2292,15 @@ class _BoundLoop(object):
             n = rng[1] - rng[0]
         if n == 0:
             return False
+        graph = _state.get('capturing')
         for m in self.mats:
             m._state = DEVICE
-            m._written()
+            m._zeroed = False
+            if graph:
+                graph.note_mat(m)
+        if self._one_record and rng is None:
+            call("op2b_launch_record", self._desc_ptr)
+            return True
         fn = self.module.fn
         if self.indirect:
             plan = self.plan
@@ -2305,7 +2318,7 @@ class _BoundLoop(object):
         else:
             call("op2b_launch_record", self._desc_ptr)
         if self.spec.mode == "lma":
-            self._reduce([m._values().ptr for m in self.mats], [zero[id(m)] for m in self.mats])
+            self._reduce([m._values().ptr for m in self.mats], zero)
         return True
 
     def _reduce(self, values, zero):
