@@ -18,6 +18,7 @@ HOST (host copy newer), DEVICE (device copy newer), BOTH.
 """
 
 import copy
+import contextlib
 import ctypes as C
 import hashlib
 import os
@@ -1788,6 +1789,33 @@ def _bind_fitting(loop, nelem=None):
         return None
 
 
+@contextlib.contextmanager
+def _stand_ins(mats):
+    """Device addresses that loops being timed write for the values of ``mats``:
+    the values themselves where all are known to be zero, zeroed again after it;
+    else memory of their size, or None if there is none.  Other threads' assembly
+    waits meanwhile: it would be timed too."""
+    with _MAT_LOCK:
+        if all(m._known_zero() for m in mats):
+            vals = [m._values() for m in mats]
+            for m in mats:
+                m._zeroed = False
+            try:
+                yield [v.ptr for v in vals]
+            finally:
+                for m, v in zip(mats, vals):
+                    v.memset(0)
+                    m._zeroed = True
+            return
+        try:
+            vals = [DeviceBuffer(m._values().nbytes) for m in mats]
+        except DeviceError as e:
+            if e.status != _lib.ERR_NOMEM:
+                raise
+            vals = []
+        yield [v.ptr for v in vals]
+
+
 class _BoundLoop(object):
     """Everything about a par_loop that does not change between calls with
     the same objects: generated stub, plan, parameter block."""
@@ -2152,18 +2180,13 @@ class _BoundLoop(object):
             bl._ready(loop)
         if sum(m.sparsity.nz for m in self.mats) == 0 or self._contributions() < _TRIAL_MIN:
             return rows
-        try:
-            stand_ins = [DeviceBuffer(m._values().nbytes) for m in self.mats]
-        except DeviceError as e:
-            if e.status != _lib.ERR_NOMEM:
-                raise
-            stand_ins = None
-        if stand_ins:
-            ms = self._device_ms(loop.args, stand_ins)
-            if rows._device_ms(loop.args, stand_ins, zero=True) < _TRIAL_ZEROED * ms:
-                if rows._device_ms(loop.args, stand_ins) >= _TRIAL_HOLDING * ms:
-                    rows._element = self
-                return rows
+        with _stand_ins(self.mats) as values:
+            if values:
+                ms = self._device_ms(loop.args, values)
+                if rows._device_ms(loop.args, values, zero=True) < _TRIAL_ZEROED * ms:
+                    if rows._device_ms(loop.args, values) >= _TRIAL_HOLDING * ms:
+                        rows._element = self
+                    return rows
         rows.row_blocks.forget(self.mats[0].sparsity)
         return self
 
@@ -2171,9 +2194,10 @@ class _BoundLoop(object):
         w = next(a for a in self.spec.args if a.kind == "mat")
         return self.nelem * w.arity * w.carity
 
-    def _device_ms(self, args, stand_ins, zero=False, enough=0.0):
-        """Device time of a run that writes ``stand_ins`` for the Mats; that of the
-        first one, which is no shorter, if it is at most ``enough`` ms."""
+    def _device_ms(self, args, values, zero=False, enough=0.0):
+        """Device time of a run that writes the addresses ``values`` for the Mats;
+        that of the first one, which is no shorter, if it is at most ``enough``
+        ms."""
         if self.consts:
             _sync_consts(self.module, self.consts)
         buf = C.create_string_buffer(self._buf.raw, self.layout.nbytes)
@@ -2181,8 +2205,8 @@ class _BoundLoop(object):
             g = args[ai].data
             g._to_device()
             struct.pack_into("<Q", buf, off, g._device.ptr)
-        for j, b in enumerate(stand_ins):
-            struct.pack_into("<Q", buf, self.layout.offset("mv%d" % j), b.ptr)
+        for j, ptr in enumerate(values):
+            struct.pack_into("<Q", buf, self.layout.offset("mv%d" % j), ptr)
             if self.row_blocks is not None:
                 struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), int(zero))
 
@@ -2190,7 +2214,7 @@ class _BoundLoop(object):
             call("op2b_launch", self.module.fn, self.grid, self.block_size, self.launch_smem, 0, buf,
                  self.layout.nbytes)
             if self.spec.mode == "lma":
-                self._reduce([b.ptr for b in stand_ins], [zero] * len(stand_ins))
+                self._reduce(values, [zero] * len(values))
 
         def timed(runs):
             e0 = Event().record()
@@ -2199,12 +2223,11 @@ class _BoundLoop(object):
             e1 = Event().record()
             e1.synchronize()
             return e0.elapsed_ms(e1) / runs
-        with _MAT_LOCK:      # other threads' assembly would be timed with it
-            first = timed(1)
-            if first <= enough:
-                return first
-            first = timed(1)
-            return first if first > _TRIAL_LONG else timed(_TRIAL_RUNS)
+        first = timed(1)
+        if first <= enough:
+            return first
+        first = timed(1)
+        return first if first > _TRIAL_LONG else timed(_TRIAL_RUNS)
 
     def _run(self, loop, rng=None):
         if self._element is not None and not all(m._known_zero() for m in self.mats):
@@ -2640,10 +2663,9 @@ def _row_blocks_or_two_phases(rows, loop):
     try:
         if 8 * added > _state['l2_bytes'] // 2:
             most = added / _LMA_PER_MS
-            stand_ins = [DeviceBuffer(m._values().nbytes) for m in rows.mats]
-            if rows._device_ms(loop.args, stand_ins, enough=most) <= most:
-                return rows
-            del stand_ins
+            with _stand_ins(rows.mats) as values:
+                if not values or rows._device_ms(loop.args, values, enough=most) <= most:
+                    return rows
         return _BoundLoop(loop, rows=False)._faster_form(rows, loop)
     except DeviceError as e:
         if e.status != _lib.ERR_NOMEM:

@@ -225,3 +225,40 @@ def test_row_blocks_within_the_second_phase_run_once(op2, monkeypatch):
     fem.assemble_p1_stiffness(op2, P)
     assert [b.spec.mode for b in bound("p1_stiff", P.elements)] == ["rowblk"]
     assert made.count("op2b_launch") == 1
+
+
+@pytest.mark.parametrize("inc_mode", ["staged", "lma"])
+@pytest.mark.parametrize("held", [False, True])
+@pytest.mark.parametrize("fails", [False, True])
+def test_timing_leaves_the_values(op2, monkeypatch, inc_mode, held, fails):
+    """Forms are timed into Mats known to be zero, which are zeroed again, but not
+    into Mats that hold values; also where the timing ends in an error."""
+    from pyop2_b200 import b200
+    from pyop2_b200.exceptions import DeviceError
+    cfg.configure(inc_mode=inc_mode, kahan=False)
+    P = problem(op2)
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 1 << 40)
+    fem.assemble_p1_stiffness(op2, P)
+    one = P.stiff.array
+    P = problem(op2)
+    if held:
+        fem.assemble_p1_stiffness(op2, P)
+    monkeypatch.setattr(b200, "_ROWBLK_MIN", 0)
+    monkeypatch.setattr(b200, "_ROWBLK_RUNS", 0)
+    monkeypatch.setattr(b200, "_TRIAL_MIN", 0)
+    b200.ParLoop._bound_cache.clear()
+    time, wrote = b200._BoundLoop._device_ms, []
+
+    def device_ms(self, args, values, *rest, **kw):
+        ms = time(self, args, values, *rest, **kw)
+        wrote.append(values == [P.stiff._values().ptr])
+        if fails:
+            raise DeviceError("no memory", 4 if inc_mode == "lma" else 2)
+        return ms
+    monkeypatch.setattr(b200._BoundLoop, "_device_ms", device_ms)
+    if fails and inc_mode == "staged":
+        with pytest.raises(DeviceError):
+            fem.assemble_p1_stiffness(op2, P)
+    fem.assemble_p1_stiffness(op2, P)
+    assert wrote and wrote == [not held] * len(wrote)
+    np.testing.assert_allclose(P.stiff.array, (2 if held else 1) * one, rtol=1e-14, atol=1e-15 * abs(one).max())
