@@ -98,6 +98,9 @@ int op2b_default_stream(uint64_t *stream);
 int op2b_stream_create(uint64_t *stream);
 int op2b_stream_destroy(uint64_t stream);
 int op2b_stream_sync(uint64_t stream);
+/* Keep the stream busy for about us microseconds (at most 1000), so that short
+ * launches issued meanwhile run back to back and can be timed. */
+int op2b_stream_pause(int32_t us, uint64_t stream);
 int op2b_device_sync(void);
 int op2b_event_create(uint64_t *event);
 int op2b_event_destroy(uint64_t event);

@@ -42,6 +42,7 @@ _SIGS = {
     "op2b_stream_create": [u64p],
     "op2b_stream_destroy": [u64],
     "op2b_stream_sync": [u64],
+    "op2b_stream_pause": [i32, u64],
     "op2b_device_sync": [],
     "op2b_event_create": [u64p],
     "op2b_event_destroy": [u64],

@@ -1272,10 +1272,17 @@ _TRIAL_MIN = 1 << 20
 # the mean of so many runs; a run of more than _TRIAL_LONG ms is long enough to be
 # told from another by itself (the Q1 stiffness above: 47 ms for both forms, not 164)
 _TRIAL_RUNS, _TRIAL_LONG = 6, 2.0
+# us in which the host issues these runs: one takes it as long as P1 256 x 256 takes
+# the GPU, and without it that loop measured 9.2 to 10.7 us in the element form and 8.3
+# to 10.4 as row blocks (8.7 to 10.4 and 8.7 with it)
+_TRIAL_PAUSE = 120
 # Of the element form's time that row blocks may take, zeroed and holding values.
 # The runs timed find in L2 what others may have driven out, and row blocks read
-# more (P1 724 x 724 holding values: 46.3 and 47.6 us, after a flush 61 and 70)
-_TRIAL_ZEROED, _TRIAL_HOLDING = 0.97, 0.9
+# more (P1 724 x 724 holding values: 46.3 and 47.6 us, after a flush 61 and 70).
+# Launches that follow one another start in steps of 2 us, which hides what short
+# runs differ by: P1 256 x 256 zeroed measures 8.7 us in either form, and takes 14.3
+# and 13.0 in a graph with its memsets and right-hand side
+_TRIAL_ZEROED, _TRIAL_HOLDING = 1.03, 0.9
 # Two-phase sums: 18.9 million contributions take op2b_lma_reduce 119 us, whatever
 # the kernel, where the contributions do not fit the L2.  Row blocks that take no
 # longer are not compared with them.
@@ -2217,6 +2224,8 @@ class _BoundLoop(object):
                 self._reduce(values, [zero] * len(values))
 
         def timed(runs):
+            if runs > 1:
+                call("op2b_stream_pause", _TRIAL_PAUSE, 0)
             e0 = Event().record()
             for _ in range(runs):
                 run()

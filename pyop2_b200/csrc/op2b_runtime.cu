@@ -283,6 +283,14 @@ static bool copy_shared(int n, const uint64_t *dst, const uint64_t *src, const u
   }
 }
 
+// One thread that counts clock cycles (2 GHz at most): work issued meanwhile runs
+// without gaps after it.  Ends after `cycles` cycles or as many looks at the clock.
+__global__ void pause_kernel(int cycles) {
+  const long long start = clock64();
+  for (int i = 0; i < cycles && clock64() - start < cycles; ++i) {
+  }
+}
+
 // Writes the smallest offending position (or INT64_MAX) to *bad.
 __global__ void map_validate_kernel(const int32_t *__restrict__ map, int64_t n, int32_t to_size,
                                     unsigned long long *bad) {
@@ -575,6 +583,13 @@ int op2b_stream_sync(uint64_t stream) {
   OP2B_REQUIRE_INIT();
   OP2B_CUDA(cudaStreamSynchronize(stream_of(stream)));
   return OP2B_OK;
+}
+
+int op2b_stream_pause(int32_t us, uint64_t stream) {
+  OP2B_REQUIRE_INIT();
+  if (us < 0 || us > 1000) return set_error(OP2B_ERR_ARG, "op2b_stream_pause: %d us (0 to 1000)", us);
+  pause_kernel<<<1, 1, 0, stream_of(stream)>>>(us * 2000);
+  return check_cuda(cudaGetLastError(), "pause_kernel");
 }
 
 int op2b_device_sync(void) {

@@ -262,3 +262,20 @@ def test_timing_leaves_the_values(op2, monkeypatch, inc_mode, held, fails):
     fem.assemble_p1_stiffness(op2, P)
     assert wrote and wrote == [not held] * len(wrote)
     np.testing.assert_allclose(P.stiff.array, (2 if held else 1) * one, rtol=1e-14, atol=1e-15 * abs(one).max())
+
+
+def test_a_pause_keeps_the_stream_busy(backend):
+    """About as long as asked (in cycles of 2 GHz); longer ones are refused."""
+    from pyop2_b200 import b200
+    from pyop2_b200._lib import call
+    from pyop2_b200.exceptions import DeviceError
+    call("op2b_stream_pause", 1, 0)
+    for us in (0, 120, 1000):
+        e0 = b200.Event().record()
+        call("op2b_stream_pause", us, 0)
+        e1 = b200.Event().record()
+        e1.synchronize()
+        assert 0.9e-3 * us <= e0.elapsed_ms(e1) < 1 + 4e-3 * us
+    for us in (-1, 1001):
+        with pytest.raises(DeviceError):
+            call("op2b_stream_pause", us, 0)
