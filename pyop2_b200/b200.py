@@ -2127,8 +2127,7 @@ class _BoundLoop(object):
                 self._ginit.append(None)
         self._gflag = [0] * len(self._gbl)
         self._mzero = [0] * len(self.mats)
-        # what is known of the Mats changes the launch; the record is all there is
-        self._uses_zero = self.row_blocks is not None or self.spec.mode == "lma"
+        # a run over the whole set is the launch record and no more
         self._one_record = not self.indirect and self.spec.mode != "lma" and self.nelem > 0
         self._written = [d for d in self.dats if any(m != "READ" for m in self.dat_access[id(d)])]
         self._reducing = [k for k, (_, _, red) in enumerate(self._gbl) if red]
@@ -2288,15 +2287,24 @@ class _BoundLoop(object):
                 self._gptr[k] = ptr
         if self.consts:
             _sync_consts(self.module, self.consts)
-        if self.mats:
+        if self._one_record and rng is None:      # the common case, without a call
+            if self.mats:
+                with _MAT_LOCK:
+                    if self.row_blocks is not None:
+                        self._pack_zero(buf)
+                    graph = _state.get('capturing')
+                    for m in self.mats:
+                        m._state = DEVICE
+                        m._zeroed = False
+                        if graph:
+                            graph.note_mat(m)
+                    call("op2b_launch_record", self._desc_ptr)
+            else:
+                call("op2b_launch_record", self._desc_ptr)
+        else:
             with _MAT_LOCK:
-                launched = self._issue(buf, rng)
-            if not launched:
-                return
-        elif self._one_record and rng is None:      # the common case, without a call
-            call("op2b_launch_record", self._desc_ptr)
-        elif not self._issue(buf, rng):
-            return
+                if not self._issue(buf, rng):
+                    return
         for d in self._written:
             d._state = DEVICE
             d._wgen += 1
@@ -2305,17 +2313,18 @@ class _BoundLoop(object):
         for k in self._reducing:
             args[self._gbl[k][1]].data._state = DEVICE
 
+    def _pack_zero(self, buf):
+        """Which Mats row blocks need not read."""
+        for j, m in enumerate(self.mats):
+            z = int(m._known_zero())
+            if z != self._mzero[j]:
+                struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), z)
+                self._mzero[j] = z
+
     def _issue(self, buf, rng):
-        """Launch what the parameter block ``buf`` describes (False: there are no
-        elements); the Mats are not known to be zero any more."""
-        if self._uses_zero:
-            zero = [m._known_zero() for m in self.mats]
-        if self.row_blocks is not None:
-            for j, z in enumerate(zero):
-                z = int(z)
-                if z != self._mzero[j]:
-                    struct.pack_into("<q", buf, self.layout.offset("mz%d" % j), z)
-                    self._mzero[j] = z
+        """Launch what the parameter block ``buf`` describes, of loops that are more
+        than one launch record (False: there are no elements); the Mats are not
+        known to be zero any more."""
         n = self.nelem
         if rng is not None:
             if self.spec.mode not in ("direct", "atomic") or rng[0] < 0 or rng[1] > \
@@ -2324,15 +2333,10 @@ class _BoundLoop(object):
             n = rng[1] - rng[0]
         if n == 0:
             return False
-        graph = _state.get('capturing')
+        zero = [m._known_zero() for m in self.mats]
         for m in self.mats:
             m._state = DEVICE
-            m._zeroed = False
-            if graph:
-                graph.note_mat(m)
-        if self._one_record and rng is None:
-            call("op2b_launch_record", self._desc_ptr)
-            return True
+            m._written()
         fn = self.module.fn
         if self.indirect:
             plan = self.plan
