@@ -707,7 +707,9 @@ class Mat(DeviceDataMixin, base.Mat):
     def zero(self):
         vals = self._vals or self._values()
         with _MAT_LOCK:
-            call("op2b_memset", vals.ptr, 0, vals.nbytes, 0)
+            rc = _lib._lib.op2b_memset(vals.ptr, 0, vals.nbytes, 0)
+            if rc:
+                _lib.check(rc, "op2b_memset")
             graph = _state.get('capturing')
             self._zeroed = graph if graph else True
             if graph:
@@ -2298,9 +2300,11 @@ class _BoundLoop(object):
                         m._zeroed = False
                         if graph:
                             graph.note_mat(m)
-                    call("op2b_launch_record", self._desc_ptr)
+                    rc = _lib._lib.op2b_launch_record(self._desc_ptr)
             else:
-                call("op2b_launch_record", self._desc_ptr)
+                rc = _lib._lib.op2b_launch_record(self._desc_ptr)
+            if rc:
+                _lib.check(rc, "op2b_launch_record")
         else:
             with _MAT_LOCK:
                 if not self._issue(buf, rng):
